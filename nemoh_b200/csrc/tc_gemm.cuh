@@ -206,13 +206,16 @@ __global__ void __launch_bounds__(128) tc_prep_wv_kernel(BatchT<float2> b, int k
   const int q = (isW ? blockIdx.x : blockIdx.x - PER) * 128 + threadIdx.x;   // < TC_T * TC_NCH
   const int ch = q / TC_T, row = q % TC_T, kb = ch * TC_KC;
   unsigned char* base = wv + blockIdx.z * TC_WV_BYTES;
+  // only the 32 x 32 blocks of the triangle are formed (W's column block, and
+  // V's row block, at most this row's); the rest of the scratch is not theirs
+  const bool held = kb / LU_NB <= row / LU_NB;
   float re[TC_KC], im[TC_KC];
   uint4 h, l;
   if (isW) {   // B column `row` of conj(W^T): conj(W[row, kb + j])
     const float2* W = P + PINV_W_OFF;
 #pragma unroll
     for (int j = 0; j < TC_KC; ++j) {
-      const float2 v = W[row + LU_OUTER * (kb + j)];
+      const float2 v = held ? W[row + LU_OUTER * (kb + j)] : make_float2(0.f, 0.f);
       re[j] = v.x;
       im[j] = v.y;
     }
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(128) tc_prep_wv_kernel(BatchT<float2> b, int k
     const float2* V = P + PINV_V_OFF;
 #pragma unroll
     for (int j = 0; j < TC_KC; ++j) {
-      const float2 v = V[(kb + j) + LU_OUTER * row];
+      const float2 v = held ? V[(kb + j) + LU_OUTER * row] : make_float2(0.f, 0.f);
       re[j] = v.x;
       im[j] = v.y;
     }
