@@ -27,6 +27,7 @@
 #include "postproc.cuh"
 #include "linalg.cuh"
 #include "mixed.cuh"
+#include "oz_gemm.cuh"
 
 using namespace nb200;
 
@@ -159,6 +160,7 @@ struct nemoh_ctx {
   DevBuf d_roff, d_rord, d_smesh, d_items, d_bnvel, d_bforce, d_reqs;
   DevBuf d_froff, d_frord, d_fx, d_fy;   // partial FP64 fallback of a ragged batch
   DevBuf d_flow;                         // workspace of the FP64 dataflow sweep
+  OzWork oz;                             // operand images of the FP64 LU's trailing updates
   long long fallback_systems = 0;         // systems re-solved with FP64 factors so far
   HostBuf h_rag, h_reqs;
   // CUDA graphs of cross-body batches (nemoh_b200_set_graphs)
@@ -347,8 +349,10 @@ int batch_capacity(nemoh_ctx* c, int nrhs, int want) {
   size_t per = (2 * cls * N * N + 2 * cls * N * (size_t)std::max(nrhs, 1)) * sizeof(double2) + sizeof(OmegaParams) +
                cls * DIAG_SCRATCH * sizeof(double2) + cls * ((N + TB - 1) / TB) * 2 * TB * TB * sizeof(double2);
   if (c->mode == NEMOH_B200_MIXED) per += mixed_bytes_per_system(N) * cls;
+  else if (N > LU_OUTER) per += oz_bytes_per_system(N) * cls;
   // existing buffers count as available
-  size_t have = c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes + c->mixed.bytes();
+  size_t have = c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes + c->mixed.bytes() +
+                c->oz.bytes();
   size_t budget = (size_t)((fr + have) * 0.8);
   // room for the Rankine caches of both depth regimes that are not allocated yet
   for (int r = 0; r < 2; ++r) {
@@ -527,9 +531,26 @@ Batch dbatch(nemoh_ctx* c, const Shape& sh) {
   return make_batch<double2>(c->d_D.as<double2>(), sh.n, c->d_diag.as<double2>(), nullptr, sh.rg);
 }
 
+// Operand images of the FP64 LU's tensor-core updates (oz_gemm.cuh) for nsys
+// systems of order up to n; false where there is no trailing update or no room
+// for them (the FP64 fallback of a mixed batch that fills the device): the
+// update then runs on the FP64 pipe.
+bool fp64_images(nemoh_ctx* c, int nsys, int n) {
+  const double rest = n - LU_OUTER;
+  if (!tc_enabled() || rest <= 0 || rest * rest * nsys < OZ_MIN_ENTRIES) return false;
+  return c->oz.ensure(nsys, n) == cudaSuccess;
+}
+
 void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
   Batch b = dbatch(c, sh);
   const int N = sh.n;
+  const bool images = fp64_images(c, nsys, N);
+  // Panel pairs are merged: after an even panel only the next panel's columns
+  // and rows are updated, the rest of the trailing matrix takes both panels'
+  // products in the next panel's update, so its bulk is read and written once
+  // per pair. deferred: the groups (by their first system) whose last panel's
+  // bulk is still to come.
+  std::map<int, bool> deferred;
   static std::atomic<unsigned long long> attr{0};
   once_per_device(attr, [] {
     CK(cudaFuncSetAttribute(zgemm_update_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -537,9 +558,29 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
   });
   lu_two_level<double2>(
       b, nsys, c->d_status.as<int>(), c->stream, c->launches,
-      [&](Batch bg, int ns, cudaStream_t sg, int, int k0, int kend) {
-        zgemm_update<double2>(bg, k0, kend - k0, Rect{kend, bg.n, kend, bg.n}, ns, sg);
-        ++c->launches;
+      [&](Batch bg, int ns, cudaStream_t sg, int s0, int k0, int kend) {
+        bool& late = deferred[s0];
+        const double rest = bg.n - kend;
+        if (!images || !(late || rest * rest * nsys >= OZ_MIN_ENTRIES)) {
+          zgemm_update<double2>(bg, k0, kend - k0, Rect{kend, bg.n, kend, bg.n}, ns, sg);
+          ++c->launches;
+          return;
+        }
+        const int set = (k0 / LU_OUTER) & 1;
+        const OzStride st = oz_stride(c->oz);
+        const OzSet cur = oz_set(c->oz, set, s0);
+        int* status = c->d_status.as<int>();
+        oz_prep(cur, st, bg, k0, ns, sg, c->launches);
+        if (late) {
+          oz_apply(cur, oz_set(c->oz, set ^ 1, s0), st, bg, k0, ns, sg, c->launches, status, TcTiles());
+          late = false;
+        } else if (kend + LU_OUTER < bg.n) {
+          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, TcTiles{0, -1, 0, 1});
+          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, TcTiles{0, 1, 1, -1});
+          late = true;
+        } else {
+          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, TcTiles());
+        }
       },
       &c->lanes, sh.rg.host_ord);
   CK(cudaGetLastError());
@@ -795,6 +836,8 @@ size_t item_bytes(const nemoh_ctx* c, const BodyState& b, int nmax, int nrhs) {
     mats += n * n * sizeof(float2);
     per_sys += nm * nrhs * (2 * sizeof(double2) + 2 * sizeof(float2)) + (DIAG_SCRATCH + PINV_SCRATCH) * sizeof(float2) +
                nblk * 2 * TB * TB * sizeof(float2) + tc_bytes_per_system(nm);
+  } else {
+    per_sys += oz_bytes_per_system(nm);
   }
   return cls * (mats + per_sys) + sizeof(OmegaParams) + sizeof(SlotMesh) + sizeof(ItemDesc);
 }
@@ -929,7 +972,11 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   const bool mixed = c->mode == NEMOH_B200_MIXED;
   const int max_it = refine_max_it(), passes = mixed ? std::min(REFINE_CHUNK, max_it) : 0;
   // the FP64 sweeps' workspace grows here, never inside a captured sequence
-  if (!mixed) fp64_sync(c, nsys, nmax);
+  // (nor the operand images of its trailing updates)
+  if (!mixed) {
+    fp64_sync(c, nsys, nmax);
+    fp64_images(c, nsys, nmax);
+  }
   // a captured sequence holds every buffer address it was captured with: the
   // key covers them all, so a buffer that moved since is captured again
   std::vector<long long> sig = {c->mode, nrhs, k, nsys, nmax, nint_max, passes, (long long)nvel_d,
@@ -942,7 +989,7 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
                                 (long long)c->mixed.inv, (long long)c->mixed.pinv, (long long)c->mixed.norms,
                                 (long long)c->mixed.state, (long long)c->mixed.tc.a, (long long)c->mixed.tc.b,
                                 (long long)c->mixed.tc.wv, (long long)c->mixed.flow, (long long)c->mixed.act,
-                                (long long)c->d_flow.p};
+                                (long long)c->d_flow.p, (long long)c->oz.a, (long long)c->oz.b, (long long)c->oz.sc};
   for (const AsmGroup& g : groups)
     sig.insert(sig.end(), {g.ninfd, g.nfd, g.n_infd, g.n_fd, (long long)g.slot_rk_infd, (long long)g.slot_rk_fd});
   sig.insert(sig.end(), ord.begin(), ord.end());
@@ -1085,7 +1132,7 @@ void solve_bodies_impl(nemoh_ctx* c, int nitem, const int* body, const double* o
   size_t fr = 0, tot = 0;
   CK(cudaMemGetInfo(&fr, &tot));
   const size_t have = c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes + c->d_diag.bytes +
-                      c->mixed.bytes();
+                      c->mixed.bytes() + c->oz.bytes();
   size_t budget = (size_t)((fr + have) * 0.8);
   // NEMOH_B200_BATCH_BYTES lowers the budget (tests use it to split a call
   // into several batches)
