@@ -26,8 +26,9 @@
 namespace nb200 {
 
 constexpr int LU_NB = 32;     // panel width
-constexpr int LU_RB = 128;    // rows per L21 CTA
-constexpr int LU_CB = 64;     // columns per U12 CTA
+constexpr int LU_PT = 256;    // threads of a panel CTA
+constexpr int LU_RB = 32;     // rows per L21 CTA
+constexpr int LU_CB = 32;     // columns per U12 CTA
 
 // A batch of systems. Uniform: every system has order n and starts `stride`
 // elements after the previous one. Ragged (systems of different bodies in one
@@ -103,66 +104,170 @@ __device__ __forceinline__ float2 cdv(float2 a, float2 b) {
 __device__ __forceinline__ double cabs2(double2 a) { return hypot(a.x, a.y); }
 __device__ __forceinline__ double cabs2(float2 a) { return hypotf(a.x, a.y); }
 
+// reciprocal of a pivot, scaled by a power of two so that |p|^2 neither
+// overflows nor underflows. Every elimination step waits for it, so 1 / d with
+// d in [1, 8) is the hardware's approximation and one Householder step (third
+// order in double precision: 2^-20 to below 2^-58; second order in single),
+// without the special cases of a general quotient.
+__device__ __forceinline__ double2 crecip(double2 p) {
+  const int e = max(__double2hiint(p.x) & 0x7ff00000, __double2hiint(p.y) & 0x7ff00000) >> 20;
+  const double s = __hiloint2double(max(1, 2046 - e) << 20, 0);
+  const double x = p.x * s, y = p.y * s, d = fma(x, x, y * y);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double h = fma(-d, r, 1.);
+  r = fma(r, fma(h, h, h), r) * s;
+  return make_double2(x * r, -y * r);
+}
+__device__ __forceinline__ float2 crecip(float2 p) {
+  const int e = max(__float_as_int(p.x) & 0x7f800000, __float_as_int(p.y) & 0x7f800000) >> 23;
+  const float s = __int_as_float(max(1, 254 - e) << 23);
+  const float x = p.x * s, y = p.y * s, d = fmaf(x, x, y * y);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(r, fmaf(-d, r, 1.f), r) * s;
+  return make_float2(x * r, -y * r);
+}
+// |p| > 1e-20 (GAUSSZ's pivot test; false for NaN); the modulus only where the
+// components' sum, at most sqrt(2) of it, does not settle it
+template <class C2>
+__device__ __forceinline__ bool pivot_ok(C2 p) {
+  return fabs(p.x) + fabs(p.y) > 1.5E-20 || cabs2(p) > 1.E-20;
+}
+__device__ __forceinline__ double2 cshfl(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ float2 cshfl(float2 v, int src) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+template <class C2>
+__device__ __forceinline__ C2 cprod(C2 a, C2 b) {
+  C2 r;
+  r.x = a.x * b.x - a.y * b.y;
+  r.y = a.x * b.y + a.y * b.x;
+  return r;
+}
+
+// Unpivoted LU of a 32 x 32 block with the inverses of both triangles, by 256
+// threads: lane = row i, warp w = columns 4 w .. 4 w + 3, everything in
+// registers. A thread's entry t of column c is a_ic while i > j, then (its
+// final value u_ic kept in `u`) the entry x_ic of inv(U), from the identity.
+// Step j:
+//   m_i = t_ij / u_jj: below the diagonal the multipliers l_ij, at and above it
+//   column j of inv(U), finished; then
+//   t_ic -= m_i u_jc (c > j)               the elimination below row j, and the
+//                                          column form of X U = I above it
+//   y_ic -= m_i y_jc (i > j, c <= j)       inv(L): the row operations on I
+// so that no lane's path depends on its row; the pivot row's entries come by
+// shuffles. The warp of columns j .. j + 3 does four steps on its own columns,
+// publishes the four vectors m and meets the others at one of eight barriers
+// (bar.sync 1 over the 256 threads); the next warp starts its four steps as soon
+// as it has applied them. The chain is the 32 reciprocals with their shuffles: a
+// barrier per step, a quotient by IEEE division and the pivot test inside the
+// chain measured 11.8 us in single and 13.9 us in double precision, this form
+// about 5 and 8 us.
+constexpr int DIAG_T = 256;
+constexpr int DIAG_W = DIAG_T / 32, DIAG_PER = LU_NB / DIAG_W;   // warps, columns per thread
+template <class C2>
+struct Diag32 {
+  C2 t[DIAG_PER], u[DIAG_PER], y[DIAG_PER];
+  // in: t the block (the identity beyond its order), y the identity; out: L below and
+  // inv(U) at and above the diagonal in t, U in u (i <= c), inv(L) in y
+  __device__ __forceinline__ C2 lu(int e, int i, int c) const { return i > c ? t[e] : u[e]; }
+  __device__ __forceinline__ C2 iu(int e, int i, int c) const { return i > c ? mkc<C2>(0., 0.) : t[e]; }
+};
+template <class C2>
+using DiagVec = C2[2][DIAG_PER][LU_NB];
+template <class C2>
+__device__ __forceinline__ void diag32(Diag32<C2>& d, int nb, DiagVec<C2>& v, int* status) {
+  const int i = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const C2 zero = mkc<C2>(0., 0.), one = mkc<C2>(1., 0.);
+  // column e of this thread beyond the pivot j: rank-1 update by m, the pivot row retired
+  auto beyond = [&](int e, int j, C2 m) {
+    const C2 u = cshfl(d.t[e], j);
+    if (i == j) {
+      d.u[e] = u;
+      d.t[e] = zero;
+    }
+    d.t[e] = cfms(d.t[e], m, u);
+  };
+  auto done = [&](int e, int j, C2 ml) { d.y[e] = cfms(d.y[e], ml, cshfl(d.y[e], j)); };
+#pragma unroll 1
+  for (int w0 = 0; w0 * DIAG_PER < nb; ++w0) {   // columns beyond nb are the identity's
+    const int j0 = w0 * DIAG_PER;
+    C2(*vb)[LU_NB] = v[w0 & 1];
+    if (w == w0) {
+#pragma unroll
+      for (int q = 0; q < DIAG_PER; ++q) {
+        const int j = j0 + q;
+        const C2 p = cshfl(d.t[q], j);
+        if (i == j) {
+          d.u[q] = p;
+          d.t[q] = one;
+        }
+        d.t[q] = cprod(d.t[q], crecip(p));
+        vb[q][i] = d.t[q];
+#pragma unroll
+        for (int e = q + 1; e < DIAG_PER; ++e) beyond(e, j, d.t[q]);
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(DIAG_T) : "memory");
+    if (w > w0) {
+#pragma unroll
+      for (int q = 0; q < DIAG_PER; ++q) {
+        const C2 m = vb[q][i];
+#pragma unroll
+        for (int e = 0; e < DIAG_PER; ++e) beyond(e, j0 + q, m);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < DIAG_PER; ++q) {
+        const C2 ml = i > j0 + q ? vb[q][i] : zero;
+#pragma unroll
+        for (int e = 0; e < DIAG_PER; ++e)
+          if (e <= q || w < w0) done(e, j0 + q, ml);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < DIAG_PER; ++e)
+    if (i == DIAG_PER * w + e && i < nb && !pivot_ok(d.u[e])) atomicCAS(status, 0, ST_PIVOT);
+}
+
 // Factor the diagonal block A11 of step k once per system (grid.z = system)
-// and invert its triangles. Scratch per system: [LU(A11) | inv(L11) | inv(U11)],
-// column-major nb x nb each (ld = nb). One thread per element of the 32 x 32
-// block, every step of the three eliminations separated by a barrier:
-//  * unpivoted Doolittle (GAUSSZ's elimination on this block): at step j the
-//    column below the pivot is divided by it, then the trailing block takes
-//    the rank-1 update;
-//  * inv(L): X = I, step j (ascending) subtracts L(i, j) X(j, :) from the rows
-//    below, the order of the column-by-column forward substitution;
-//  * inv(U): X = I, step j (descending) divides row j by U(j, j) and
-//    subtracts U(i, j) X(j, :) from the rows above.
-// With b.pinv (two-level LU) inv(L) also goes to the slot of this block in the
-// current outer panel. (Measured against two 128-thread forms, warp-owned
-// columns with the inverses either by warp-owned columns or one column per
-// lane in registers: 28.6 us per launch here against 78.5 and 65 us; the
-// register form's long unrolled instruction stream stalls on instruction
-// fetch.)
-constexpr int LU_DIAG_THREADS = LU_NB * LU_NB;
+// and invert its triangles (diag32). Scratch per system: [LU(A11) | inv(L11) |
+// inv(U11)], column-major nb x nb each (ld = nb). With b.pinv (two-level LU)
+// inv(L) also goes to the slot of this block in the current outer panel.
+// Latency of one CTA per system, 32 dependent steps: 8.2 us per launch in single
+// and 12.3 us in double precision (14.4 and 17.9 us with a barrier per step).
+constexpr int LU_DIAG_THREADS = DIAG_T;
 template <class C2>
 __global__ void __launch_bounds__(LU_DIAG_THREADS) lu_diag_kernel(BatchT<C2> b, int k, int* status) {
-  __shared__ C2 sb[LU_NB * LU_NB];   // the block, column-major, ld = nb
-  __shared__ C2 xl[LU_NB * LU_NB];   // inv(L11), ld = LU_NB
-  __shared__ C2 xu[LU_NB * LU_NB];   // inv(U11), ld = LU_NB
+  __shared__ DiagVec<C2> v;
   const int n = b.order(blockIdx.z);
   if (k >= n) return;
   const int nb = min(LU_NB, n - k);
-  const int i = threadIdx.x & (LU_NB - 1), c = threadIdx.x / LU_NB;
-  const bool in = i < nb && c < nb;
+  const int i = threadIdx.x & 31, w = threadIdx.x >> 5;
   const C2* A = b.sys(blockIdx.z);
-  if (in) sb[i + nb * c] = A[(k + i) + (long long)n * (k + c)];
-  __syncthreads();
-  for (int j = 0; j < nb; ++j) {
-    if (threadIdx.x == 0 && !(cabs2(sb[j + nb * j]) > 1.E-20)) atomicCAS(status, 0, ST_PIVOT);
-    if (in && c == j && i > j) sb[i + nb * j] = cdv(sb[i + nb * j], sb[j + nb * j]);
-    __syncthreads();
-    if (in && i > j && c > j) sb[i + nb * c] = cfms(sb[i + nb * c], sb[i + nb * j], sb[j + nb * c]);
-    __syncthreads();
+  Diag32<C2> d;
+#pragma unroll
+  for (int e = 0; e < DIAG_PER; ++e) {
+    const int c = DIAG_PER * w + e;
+    const C2 id = mkc<C2>(i == c ? 1. : 0., 0.);
+    d.t[e] = i < nb && c < nb ? A[(k + i) + (long long)n * (k + c)] : id;
+    d.y[e] = d.u[e] = id;
   }
-  const C2 one = mkc<C2>(1., 0.), zero = mkc<C2>(0., 0.);
-  if (in) {
-    xl[i + LU_NB * c] = i == c ? one : zero;
-    xu[i + LU_NB * c] = i == c ? one : zero;
-  }
-  __syncthreads();
-  for (int step = 0; step < nb; ++step) {
-    const int jl = step, ju = nb - 1 - step;
-    if (in && i == ju && c >= ju) xu[ju + LU_NB * c] = cdv(xu[ju + LU_NB * c], sb[ju + nb * ju]);
-    __syncthreads();
-    if (in && i > jl && c <= jl) xl[i + LU_NB * c] = cfms(xl[i + LU_NB * c], sb[i + nb * jl], xl[jl + LU_NB * c]);
-    if (in && i < ju && c >= ju) xu[i + LU_NB * c] = cfms(xu[i + LU_NB * c], sb[i + nb * ju], xu[ju + LU_NB * c]);
-    __syncthreads();
-  }
+  diag32(d, nb, v, status);
   C2* D = b.diag + (long long)blockIdx.z * DIAG_SCRATCH;
   C2* P = b.pinv ? b.pinv + (long long)blockIdx.z * PINV_SCRATCH + ((k % LU_OUTER) / LU_NB) * LU_NB * LU_NB : nullptr;
-  if (in) {
-    const int q = i + nb * c;
-    D[q] = sb[q];
-    D[LU_NB * LU_NB + q] = xl[i + LU_NB * c];
-    D[2 * LU_NB * LU_NB + q] = xu[i + LU_NB * c];
-    if (P) P[q] = xl[i + LU_NB * c];
+#pragma unroll
+  for (int e = 0; e < DIAG_PER; ++e) {
+    const int c = DIAG_PER * w + e, q = i + nb * c;
+    if (i >= nb || c >= nb) continue;
+    D[q] = d.lu(e, i, c);
+    D[LU_NB * LU_NB + q] = d.y[e];
+    D[2 * LU_NB * LU_NB + q] = d.iu(e, i, c);
+    if (P) P[q] = d.y[e];
   }
 }
 
@@ -191,15 +296,19 @@ __device__ __forceinline__ void cmac(C2& acc, C2 a, C2 b) {
   acc.y = fmx(a.y, b.x, acc.y);
 }
 
-// L21 <- A21 inv(U11) (CTAs [0, nrb), one thread per row) and
-// U12 <- inv(L11) A12 for the columns [k + nb, ucol_end) (CTAs [nrb, nrb+ncb),
-// one lane per row of a column), with the
-// inverses from lu_diag_kernel; CTA 0 also stores the factored A11 into A
+// L21 <- A21 inv(U11) (CTAs [0, nrb), 32 rows each) and U12 <- inv(L11) A12 for
+// the columns [k + nb, ucol_end) (CTAs [nrb, nrb + ncb), 32 columns each), with
+// the inverses from lu_diag_kernel; CTA 0 also stores the factored A11 into A
 // (no kernel of the step reads A11 from A). Launch with at least one CTA.
+// Both are a 32 x 32 tile times a 32 x 32 triangle held in shared memory: a
+// thread owns one row and four columns of the tile (columns warp, warp + 8,
+// ...), so one lane-consecutive load and up to four broadcast ones serve four
+// complex FMAs, and the triangle's zero half is skipped. The 32-row split
+// spreads a panel over four times the CTAs of a row per thread.
 template <class C2>
-__global__ void __launch_bounds__(LU_RB) lu_panel_kernel(BatchT<C2> b, int k, int ucol_end) {
-  __shared__ C2 inv[LU_NB * LU_NB];
-  __shared__ C2 work[LU_NB * LU_CB];
+__global__ void __launch_bounds__(LU_PT) lu_panel_kernel(BatchT<C2> b, int k, int ucol_end) {
+  __shared__ C2 inv[LU_NB * LU_NB];    // inv(U11) or inv(L11), column-major
+  __shared__ C2 work[LU_NB * LU_NB];   // the tile, column-major: (row, j) of A21 or (j, column) of A12
   const int n = b.order(blockIdx.z);
   if (k >= n) return;
   ucol_end = min(ucol_end, n);
@@ -208,46 +317,47 @@ __global__ void __launch_bounds__(LU_RB) lu_panel_kernel(BatchT<C2> b, int k, in
   const C2* D = b.diag + (long long)blockIdx.z * DIAG_SCRATCH;
   const int rest = n - k - nb;
   const int nrb = (rest + LU_RB - 1) / LU_RB;
+  const C2 zero = mkc<C2>(0., 0.);
   if (blockIdx.x == 0)
-    for (int q = threadIdx.x; q < nb * nb; q += blockDim.x) A[(k + q % nb) + (long long)n * (k + q / nb)] = D[q];
-  if (blockIdx.x < nrb) {
-    for (int q = threadIdx.x; q < nb * nb; q += blockDim.x) inv[q] = D[2 * LU_NB * LU_NB + q];
-    __syncthreads();
-    const int r = k + nb + blockIdx.x * LU_RB + threadIdx.x;
-    if (r >= n) return;
-    C2 x[LU_NB];
+    for (int q = threadIdx.x; q < nb * nb; q += LU_PT) A[(k + q % nb) + (long long)n * (k + q / nb)] = D[q];
+  const bool lower = (int)blockIdx.x < nrb;   // this CTA's product: L21 or U12
+  const int r0 = lower ? k + nb + blockIdx.x * LU_RB : k;
+  const int c0 = lower ? k : k + nb + ((int)blockIdx.x - nrb) * LU_CB;
+  const int nr = lower ? min(LU_RB, n - r0) : nb, nc = lower ? nb : min(LU_CB, ucol_end - c0);
+  if (nr <= 0 || nc <= 0) return;
+  const C2* T = D + (lower ? 2 : 1) * LU_NB * LU_NB;
 #pragma unroll
-    for (int c = 0; c < LU_NB; ++c)
-      x[c] = (c < nb) ? A[r + (long long)n * (k + c)] : mkc<C2>(0., 0.);
-    // out(c) = sum_{j <= c} x(j) invU(j, c)
-#pragma unroll
-    for (int c = 0; c < LU_NB; ++c) {
-      if (c < nb) {
-        C2 acc = mkc<C2>(0., 0.);
-#pragma unroll
-        for (int j = 0; j <= c; ++j) cmac(acc, x[j], inv[j + nb * c]);
-        A[r + (long long)n * (k + c)] = acc;
-      }
-    }
-    return;
-  }
-  for (int q = threadIdx.x; q < nb * nb; q += blockDim.x) inv[q] = D[LU_NB * LU_NB + q];
-  const int c0 = k + nb + (blockIdx.x - nrb) * LU_CB;
-  const int ncol = min(LU_CB, ucol_end - c0);
-  for (int q = threadIdx.x; q < nb * ncol; q += blockDim.x) {
-    const int i = q % nb, c = q / nb;
-    work[i + nb * c] = A[(k + i) + (long long)n * (c0 + c)];
+  for (int q = threadIdx.x; q < LU_NB * LU_NB; q += LU_PT) {
+    const int i = q % LU_NB, c = q / LU_NB;
+    inv[q] = i < nb && c < nb ? T[i + nb * c] : zero;
+    work[q] = i < nr && c < nc ? A[(r0 + i) + (long long)n * (c0 + c)] : zero;
   }
   __syncthreads();
-  // y(i, c) = a(i, c) + sum_{j < i} invL(i, j) a(j, c): lane = row i, the
-  // CTA's four warps take every fourth column; results go straight to A
-  const int i = threadIdx.x & 31;
-  if (i >= nb) return;
-  for (int c = threadIdx.x >> 5; c < ncol; c += LU_RB / 32) {
-    const C2* a = work + nb * c;
-    C2 acc = a[i];
-    for (int j = 0; j < i; ++j) cmac(acc, inv[i + nb * j], a[j]);
-    A[(k + i) + (long long)n * (c0 + c)] = acc;
+  const int i = threadIdx.x & (LU_NB - 1), w = threadIdx.x / LU_NB;
+  constexpr int W = LU_PT / LU_NB, PER = LU_NB / W;
+  C2 acc[PER];
+#pragma unroll
+  for (int m = 0; m < PER; ++m) acc[m] = zero;
+  if (lower) {
+#pragma unroll 8
+    for (int j = 0; j < LU_NB; ++j) {
+      const C2 x = work[i + LU_NB * j];
+#pragma unroll
+      for (int m = 0; m < PER; ++m)
+        if (j <= w + W * m) cmac(acc[m], x, inv[j + LU_NB * (w + W * m)]);
+    }
+  } else {
+#pragma unroll 8
+    for (int j = 0; j < LU_NB; ++j) {
+      const C2 x = inv[i + LU_NB * j];   // zero for j > i
+#pragma unroll
+      for (int m = 0; m < PER; ++m) cmac(acc[m], x, work[j + LU_NB * (w + W * m)]);
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {
+    const int c = w + W * m;
+    if (i < nr && c < nc) A[(r0 + i) + (long long)n * (c0 + c)] = acc[m];
   }
 }
 
@@ -365,9 +475,77 @@ __global__ void __launch_bounds__(128) zgemm_update_kernel(BatchT<C2> b, int k, 
   }
 }
 
+// The same update by 32 x 32 tiles, inner dimension in chunks of 32 held whole in
+// shared memory: thread = one row, four columns. A 64 x 64 tile keeps its one
+// warp per scheduler waiting on its chunks and takes 39 us at least for K = 128;
+// this form gives four times the CTAs, six to an SM. FP64, K = 128, us against
+// the 64 x 64 tiles: 12 / 39 for one system of 300, 59 / 63 for four of 600, 351
+// / 351 for ten of 900 (5,760 tiles), 867 / 799 for ten of 1,400; K = 32, twenty
+// systems of 1,200: 35 / 64 inside the panel, 33 / 52 for its row strip.
+constexpr int GS_T = 32, GS_THREADS = 256, GS_W = GS_THREADS / 32;
+constexpr long long GS_MAX_CTAS = 5000;
+template <class C2>
+__global__ void __launch_bounds__(GS_THREADS) zgemm_small_kernel(BatchT<C2> b, int k, int kb, Rect rc) {
+  __shared__ C2 As[GS_T * GS_T];   // column-major: (row, kk)
+  __shared__ C2 Bs[GS_T * GS_T];   // column-major: (kk, column)
+  const int n = b.order(blockIdx.z);
+  rc.r1 = min(rc.r1, n);
+  rc.c1 = min(rc.c1, n);
+  kb = min(kb, n - k);
+  const int r0 = rc.r0 + blockIdx.y * GS_T, c0 = rc.c0 + blockIdx.x * GS_T;
+  if (r0 >= rc.r1 || c0 >= rc.c1 || kb <= 0) return;
+  C2* A = b.sys(blockIdx.z);
+  const int i = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r = r0 + i;
+  constexpr int PER = GS_T / GS_W;
+  // the products are summed apart from the tile and subtracted once: summed
+  // onto it, every FMA would round at the tile's magnitude
+  C2 acc[PER], cur[PER];
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {   // the tile itself: in flight while the operands load
+    const int c = c0 + w + GS_W * m;
+    acc[m] = mkc<C2>(0., 0.);
+    cur[m] = r < rc.r1 && c < rc.c1 ? A[r + (long long)n * c] : acc[m];
+  }
+  for (int k0 = 0; k0 < kb; k0 += GS_T) {
+    const int kc = min(GS_T, kb - k0);
+    if (k0 > 0) __syncthreads();
+#pragma unroll
+    for (int m = 0; m < PER; ++m) {
+      const int kk = w + GS_W * m;   // column of the A tile, column of the B tile
+      const bool va = r < rc.r1 && kk < kc, vb = c0 + kk < rc.c1 && i < kc;
+      cp_async_elem(As + i + GS_T * kk, va ? A + r + (long long)n * (k + k0 + kk) : A, va);
+      cp_async_elem(Bs + i + GS_T * kk, vb ? A + (k + k0 + i) + (long long)n * (c0 + kk) : A, vb);
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll 4
+    for (int kk = 0; kk < GS_T; ++kk) {
+      const C2 a = As[i + GS_T * kk];
+#pragma unroll
+      for (int m = 0; m < PER; ++m) cmac(acc[m], a, Bs[kk + GS_T * (w + GS_W * m)]);
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < PER; ++m) {
+    const int c = c0 + w + GS_W * m;
+    if (r < rc.r1 && c < rc.c1) {
+      cur[m].x -= acc[m].x;
+      cur[m].y -= acc[m].y;
+      A[r + (long long)n * c] = cur[m];
+    }
+  }
+}
+
 template <class C2>
 inline void zgemm_update(BatchT<C2> b, int k, int kb, Rect rc, int nsys, cudaStream_t st) {
   if (rc.r1 <= rc.r0 || rc.c1 <= rc.c0) return;
+  const long long small = (long long)((rc.c1 - rc.c0 + GS_T - 1) / GS_T) * ((rc.r1 - rc.r0 + GS_T - 1) / GS_T) * nsys;
+  if (kb <= GS_T || small <= GS_MAX_CTAS) {
+    zgemm_small_kernel<C2><<<dim3((rc.c1 - rc.c0 + GS_T - 1) / GS_T, (rc.r1 - rc.r0 + GS_T - 1) / GS_T, nsys), GS_THREADS, 0,
+                             st>>>(b, k, kb, rc);
+    return;
+  }
   const dim3 grid((rc.c1 - rc.c0 + GM_T - 1) / GM_T, (rc.r1 - rc.r0 + GM_T - 1) / GM_T, nsys);
   zgemm_update_kernel<C2><<<grid, 128, zgemm_smem<C2>(), st>>>(b, k, kb, rc);
 }
@@ -466,17 +644,30 @@ __global__ void __launch_bounds__(128) strip_kernel(BatchT<C2> b, int k0) {
 // strip's blocks no longer wait on one another, so every block of W a CTA
 // needs can be in flight at once.
 //
-// strip_winv_kernel: one CTA per system, thread = element (r, c) of a 32 x 32
-// block. Column block j of W: W_jj = inv(L_jj) (from lu_diag), then for the
-// blocks below W_ij = -inv(L_ii) sum_{k=j}^{i-1} L_ik W_kj.
+// A column block j of W: W_jj = inv(L_jj) (from lu_diag), then for the blocks
+// below W_ij = -inv(L_ii) sum_{k=j}^{i-1} L_ik W_kj. The column blocks do not
+// depend on one another, so each has a CTA; thread = row r, columns cg + 8 m of
+// a 32 x 32 block (one lane-consecutive load per four complex FMAs).
 constexpr int SW_BLK = LU_OUTER / LU_NB;
+constexpr int PI_THREADS = 256;
+constexpr int PI_CG = PI_THREADS / LU_NB, PI_PER = LU_NB / PI_CG;
 template <class C2>
 constexpr int strip_winv_smem() {   // a column block of W, the sum S, the L11 blocks below the diagonal, inv(L_ii)
   return (SW_BLK * LU_NB * LU_NB + LU_NB * LU_NB + (SW_BLK * (SW_BLK - 1) / 2) * LU_NB * LU_NB +
           SW_BLK * LU_NB * LU_NB) * (int)sizeof(C2);
 }
+// acc (this thread's four entries) += a b for 32 x 32 column-major blocks
 template <class C2>
-__device__ __forceinline__ void strip_winv_body(const BatchT<C2>& b, int k0) {
+__device__ __forceinline__ void blk_mac(C2* acc, const C2* a, const C2* b, int r, int cg) {
+#pragma unroll 8
+  for (int m = 0; m < LU_NB; ++m) {
+    const C2 x = a[r + LU_NB * m];
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) cmac(acc[q], x, b[m + LU_NB * (cg + PI_CG * q)]);
+  }
+}
+template <class C2>
+__device__ __forceinline__ void strip_winv_body(const BatchT<C2>& b, int k0, int j) {
   extern __shared__ __align__(16) unsigned char sw_sm[];
   constexpr int BB = LU_NB * LU_NB;
   C2* Wc = reinterpret_cast<C2*>(sw_sm);   // [SW_BLK][BB] column block j of W, column-major blocks
@@ -488,35 +679,47 @@ __device__ __forceinline__ void strip_winv_body(const BatchT<C2>& b, int k0) {
   const C2* A = b.sys(blockIdx.z);
   const C2* P = b.pinv + (long long)blockIdx.z * PINV_SCRATCH;
   C2* W = b.pinv + (long long)blockIdx.z * PINV_SCRATCH + PINV_W_OFF;
-  const int r = threadIdx.x % LU_NB, c = threadIdx.x / LU_NB, e = r + LU_NB * c;
-  // every block this system needs, loaded once (coalesced along the rows)
-  for (int i = 1; i < SW_BLK; ++i)
-    for (int k = 0; k < i; ++k)
-      Ls[((i * (i - 1)) / 2 + k) * BB + e] = A[(k0 + i * LU_NB + r) + (long long)n * (k0 + k * LU_NB + c)];
-  for (int i = 0; i < SW_BLK; ++i) Ps[i * BB + e] = P[i * BB + e];
-  for (int j = 0; j < SW_BLK; ++j) {
-    __syncthreads();   // the staged blocks (first pass) and the previous column block's stores are done
-    Wc[j * BB + e] = Ps[j * BB + e];
-    for (int i = j + 1; i < SW_BLK; ++i) {
-      __syncthreads();   // W_kj for k < i are in shared memory
-      C2 acc = mkc<C2>(0., 0.);
-      for (int k = j; k < i; ++k) {
-        const C2* L = Ls + ((i * (i - 1)) / 2 + k) * BB + r;
-        const C2* Wk = Wc + k * BB + LU_NB * c;
-#pragma unroll 8
-        for (int m = 0; m < LU_NB; ++m) cmac(acc, L[LU_NB * m], Wk[m]);
+  const int r = threadIdx.x % LU_NB, cg = threadIdx.x / LU_NB;
+  // every block this column block needs, loaded once (coalesced along the rows)
+  for (int i = j + 1; i < SW_BLK; ++i)
+    for (int k = j; k < i; ++k)
+#pragma unroll
+      for (int q = 0; q < PI_PER; ++q) {
+        const int c = cg + PI_CG * q;
+        Ls[((i * (i - 1)) / 2 + k) * BB + r + LU_NB * c] = A[(k0 + i * LU_NB + r) + (long long)n * (k0 + k * LU_NB + c)];
       }
-      S[e] = acc;
-      __syncthreads();
-      const C2* Pi = Ps + i * BB + r;
-      C2 w = mkc<C2>(0., 0.);
-#pragma unroll 8
-      for (int m = 0; m < LU_NB; ++m) cmac(w, Pi[LU_NB * m], S[m + LU_NB * c]);
-      Wc[i * BB + e] = mkc<C2>(-w.x, -w.y);
+  for (int i = j; i < SW_BLK; ++i)
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) {
+      const int e = r + LU_NB * (cg + PI_CG * q);
+      Ps[i * BB + e] = P[i * BB + e];
     }
-    __syncthreads();
-    for (int i = j; i < SW_BLK; ++i) W[(i * LU_NB + r) + LU_OUTER * (j * LU_NB + c)] = Wc[i * BB + e];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PI_PER; ++q) {
+    const int e = r + LU_NB * (cg + PI_CG * q);
+    Wc[j * BB + e] = Ps[j * BB + e];
   }
+  for (int i = j + 1; i < SW_BLK; ++i) {
+    __syncthreads();   // W_kj for k < i are in shared memory
+    C2 acc[PI_PER], v[PI_PER];
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) acc[q] = v[q] = mkc<C2>(0., 0.);
+    for (int k = j; k < i; ++k) blk_mac(acc, Ls + ((i * (i - 1)) / 2 + k) * BB, Wc + k * BB, r, cg);
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) S[r + LU_NB * (cg + PI_CG * q)] = acc[q];
+    __syncthreads();
+    blk_mac(v, Ps + i * BB, S, r, cg);
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) Wc[i * BB + r + LU_NB * (cg + PI_CG * q)] = mkc<C2>(-v[q].x, -v[q].y);
+  }
+  __syncthreads();
+  for (int i = j; i < SW_BLK; ++i)
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) {
+      const int c = cg + PI_CG * q;
+      W[(i * LU_NB + r) + LU_OUTER * (j * LU_NB + c)] = Wc[i * BB + r + LU_NB * c];
+    }
 }
 
 // strip_gemm_kernel: CTA = one system and ST_C columns of the strip (held in
@@ -606,80 +809,163 @@ __device__ __forceinline__ void strip_gemm_body(const BatchT<C2>& b, int k0, int
 // then the outer update as before.
 // ---------------------------------------------------------------------------
 template <class C2>
-constexpr int panel_block_smem() {   // the block, then one 32 x 32 scratch per triangle inversion
-  return (LU_OUTER * LU_OUTER + 2 * SW_BLK * LU_NB * LU_NB) * (int)sizeof(C2);
+constexpr int panel_block_smem() {   // the block, inv(L_jj), inv(U_jj)
+  return (LU_OUTER * LU_OUTER + 2 * LU_NB * LU_NB) * (int)sizeof(C2);
+}
+// Right-looking over the 32 x 32 diagonal blocks: diag32 factors block bi and
+// inverts its triangles in registers, then L_ij = A_ij inv(U_jj) below it (half
+// the warps) and U_ji = inv(L_jj) A_ji right of it (the other half), and the
+// rest of the block takes the rank-32 update; lane = row, a warp owns whole
+// columns, up to 3 x 3 entries per thread, two k per 16-byte broadcast load. An
+// element-by-element elimination of the whole block reads and writes the block
+// once per step and is bound by shared memory: 170-240 us per launch in a barge
+// step, 55 us in this form (a lone launch; 4 diag32, 0.27 M complex FMAs each way
+// through shared memory, and the block's way in and out).
+template <class C2, int G>
+__device__ __forceinline__ void block_step(C2* T, const C2* Ps, const C2* Qs, int o) {
+  constexpr int LD = LU_OUTER, HW = 16;   // warps of each product
+  const int i = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int e = o + LU_NB;                // rows and columns beyond the block: e + 32 m
+  const C2 zero = mkc<C2>(0., 0.);
+  C2 z[2 * G];
+#pragma unroll
+  for (int m = 0; m < 2 * G; ++m) z[m] = zero;
+  if (w < HW) {   // L(e + 32 m + i, o + w + 16 h)
+#pragma unroll 4
+    for (int j = 0; j < LU_NB; j += 2) {
+      C2 q[2][2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) ld_pair(Qs + j + LU_NB * (w + HW * h), q[h][0], q[h][1]);
+#pragma unroll
+      for (int m = 0; m < G; ++m) {
+        const C2 x0 = T[(e + LU_NB * m + i) + LD * (o + j)], x1 = T[(e + LU_NB * m + i) + LD * (o + j + 1)];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          cmac(z[2 * m + h], x0, q[h][0]);
+          cmac(z[2 * m + h], x1, q[h][1]);
+        }
+      }
+    }
+  } else {        // U(o + i, e + (w - 16) + 16 m)
+    const int c = e + w - HW;
+#pragma unroll 4
+    for (int j = 0; j < LU_NB; j += 2) {
+      const C2 p0 = Ps[i + LU_NB * j], p1 = Ps[i + LU_NB * (j + 1)];
+#pragma unroll
+      for (int m = 0; m < 2 * G; ++m) {
+        C2 y0, y1;
+        ld_pair(T + (o + j) + LD * (c + HW * m), y0, y1);
+        cmac(z[m], p0, y0);
+        cmac(z[m], p1, y1);
+      }
+    }
+  }
+  __syncthreads();   // every thread has read the old blocks
+  if (w < HW) {
+#pragma unroll
+    for (int m = 0; m < G; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) T[(e + LU_NB * m + i) + LD * (o + w + HW * h)] = z[2 * m + h];
+  } else {
+#pragma unroll
+    for (int m = 0; m < 2 * G; ++m) T[(o + i) + LD * (e + w - HW + HW * m)] = z[m];
+  }
+  __syncthreads();
+  C2 acc[G][G];
+#pragma unroll
+  for (int m = 0; m < G; ++m)
+#pragma unroll
+    for (int q = 0; q < G; ++q) acc[m][q] = zero;
+#pragma unroll 2
+  for (int j = 0; j < LU_NB; j += 2) {
+    C2 y[G][2];
+#pragma unroll
+    for (int q = 0; q < G; ++q) ld_pair(T + (o + j) + LD * (e + LU_NB * q + w), y[q][0], y[q][1]);
+#pragma unroll
+    for (int m = 0; m < G; ++m) {
+      const C2 x0 = T[(e + LU_NB * m + i) + LD * (o + j)], x1 = T[(e + LU_NB * m + i) + LD * (o + j + 1)];
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        cmac(acc[m][q], x0, y[q][0]);
+        cmac(acc[m][q], x1, y[q][1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < G; ++m)
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      C2& v = T[(e + LU_NB * m + i) + LD * (e + LU_NB * q + w)];
+      v.x -= acc[m][q].x;
+      v.y -= acc[m][q].y;
+    }
+  __syncthreads();
 }
 template <class C2>
 __global__ void __launch_bounds__(1024) panel_block_kernel(BatchT<C2> b, int k0, int* status) {
   extern __shared__ __align__(16) unsigned char pb_sm[];
+  __shared__ DiagVec<C2> dv;
   C2* T = reinterpret_cast<C2*>(pb_sm);   // [LU_OUTER][LU_OUTER] column-major
-  C2* X = T + LU_OUTER * LU_OUTER;        // [2 * SW_BLK][LU_NB][LU_NB] inversion scratch
+  C2* Ps = T + LU_OUTER * LU_OUTER;       // inv(L_jj), inv(U_jj), column-major
+  C2* Qs = Ps + LU_NB * LU_NB;
   const int n = b.order(blockIdx.z);
   if (k0 >= n) return;
   const int nb = min(LU_OUTER, n - k0), t = threadIdx.x;
+  const int i = t & (LU_NB - 1), w = t / LU_NB;
+  constexpr int LD = LU_OUTER, NBLK = LU_OUTER / LU_NB;
+  static_assert(NBLK == 4, "the steps below are written out for four diagonal blocks");
+  const C2 zero = mkc<C2>(0., 0.);
   C2* A = b.sys(blockIdx.z);
-  for (int q = t; q < LU_OUTER * LU_OUTER; q += blockDim.x) {
-    const int r = q % LU_OUTER, c = q / LU_OUTER;
-    T[q] = (r < nb && c < nb) ? A[(k0 + r) + (long long)n * (k0 + c)] : mkc<C2>(0., 0.);
+  C2* P = b.pinv + (long long)blockIdx.z * PINV_SCRATCH;
+#pragma unroll 8
+  for (int q = t; q < LD * LD; q += 1024) {   // zeros beyond nb: the products there stay zero
+    const int r = q % LD, c = q / LD;
+    T[q] = (r < nb && c < nb) ? A[(k0 + r) + (long long)n * (k0 + c)] : zero;
   }
   __syncthreads();
-  // thread = (row tr, every eighth column from tc0): the row's multiplier is
-  // read once per step, the pivot row's entries are broadcast within a warp
-  const int tr = t % LU_OUTER, tc0 = t / LU_OUTER;
-  constexpr int CSTEP = 1024 / LU_OUTER;
-  for (int j = 0; j < nb; ++j) {
-    if (t == 0 && !(cabs2(T[j + LU_OUTER * j]) > 1.E-20)) atomicCAS(status, 0, ST_PIVOT);
-    if (t > j && t < nb) T[t + LU_OUTER * j] = cdv(T[t + LU_OUTER * j], T[j + LU_OUTER * j]);
-    __syncthreads();
-    if (tr > j && tr < nb) {
-      const C2 l = T[tr + LU_OUTER * j];
-      for (int c = j + 1 + tc0; c < nb; c += CSTEP)
-        T[tr + LU_OUTER * c] = cfms(T[tr + LU_OUTER * c], l, T[j + LU_OUTER * c]);
-    }
-    __syncthreads();
-  }
-  for (int q = t; q < LU_OUTER * LU_OUTER; q += blockDim.x) {
-    const int r = q % LU_OUTER, c = q / LU_OUTER;
-    if (r < nb && c < nb) A[(k0 + r) + (long long)n * (k0 + c)] = T[q];
-  }
-  // inverses of the diagonal blocks' triangles: task = (triangle, block), one
-  // thread per column of the inverse; a partial last block keeps the
-  // identity beyond nb (those rows and columns are never used)
-  C2* P = b.pinv + (long long)blockIdx.z * PINV_SCRATCH;
-  const int task = t / 128, col = t % 128;
-  if (col < LU_NB) {
-    const bool upper = task >= SW_BLK;
-    const int bi = task % SW_BLK, o = bi * LU_NB;
-    C2* x = X + task * LU_NB * LU_NB + LU_NB * col;   // this column, in shared memory
-    const int nbb = max(0, min(LU_NB, nb - o));
-    for (int i = 0; i < LU_NB; ++i) x[i] = mkc<C2>(i == col ? 1. : 0., 0.);
-    if (col < nbb) {
-      if (!upper) {   // unit lower: x_i = -sum_{k=col}^{i-1} L_ik x_k
-        for (int i = col + 1; i < nbb; ++i) {
-          C2 v = mkc<C2>(0., 0.);
-          for (int k = col; k < i; ++k) cmac(v, T[(o + i) + LU_OUTER * (o + k)], x[k]);
-          x[i] = mkc<C2>(-v.x, -v.y);
-        }
-      } else {        // upper: x_col = 1 / U_cc, x_i = -(sum_{k=i+1}^{col} U_ik x_k) / U_ii
-        x[col] = cdv(mkc<C2>(1., 0.), T[(o + col) + LU_OUTER * (o + col)]);
-        for (int i = col - 1; i >= 0; --i) {
-          C2 v = mkc<C2>(0., 0.);
-          for (int k = i + 1; k <= col; ++k) cmac(v, T[(o + i) + LU_OUTER * (o + k)], x[k]);
-          const C2 d = cdv(v, T[(o + i) + LU_OUTER * (o + i)]);
-          x[i] = mkc<C2>(-d.x, -d.y);
-        }
+#pragma unroll 1
+  for (int bi = 0; bi < NBLK; ++bi) {
+    const int o = bi * LU_NB, nbb = max(0, min(LU_NB, nb - o));
+    if (t < DIAG_T) {
+      // a partial last block keeps the identity beyond nb (rows and columns never used)
+      Diag32<C2> d;
+#pragma unroll
+      for (int m = 0; m < DIAG_PER; ++m) {
+        const int c = DIAG_PER * w + m;
+        const C2 id = mkc<C2>(i == c ? 1. : 0., 0.);
+        d.t[m] = i < nbb && c < nbb ? T[(o + i) + LD * (o + c)] : id;
+        d.y[m] = d.u[m] = id;
+      }
+      diag32(d, nbb, dv, status);
+#pragma unroll
+      for (int m = 0; m < DIAG_PER; ++m) {
+        const int c = DIAG_PER * w + m, q = i + LU_NB * c;
+        const C2 x = d.iu(m, i, c);
+        if (i < nbb && c < nbb) T[(o + i) + LD * (o + c)] = d.lu(m, i, c);
+        Ps[q] = d.y[m];
+        Qs[q] = x;
+        P[bi * LU_NB * LU_NB + q] = d.y[m];
+        P[PINV_Q_OFF + bi * LU_NB * LU_NB + q] = x;
       }
     }
-    C2* dst = P + (upper ? PINV_Q_OFF : 0) + bi * LU_NB * LU_NB + LU_NB * col;
-    for (int i = 0; i < LU_NB; ++i) dst[i] = x[i];
+    __syncthreads();
+    if (o + LU_NB >= nb) continue;   // uniform; the blocks beyond nb still write their identities
+    if (bi == 0) block_step<C2, 3>(T, Ps, Qs, o);
+    else if (bi == 1) block_step<C2, 2>(T, Ps, Qs, o);
+    else block_step<C2, 1>(T, Ps, Qs, o);
+  }
+#pragma unroll 8
+  for (int q = t; q < LD * LD; q += 1024) {
+    const int r = q % LD, c = q / LD;
+    if (r < nb && c < nb) A[(k0 + r) + (long long)n * (k0 + c)] = T[q];
   }
 }
 
 // V = inv(U11) of the panel from the blocks of U11 (in A) and Q: column block
 // j of V: V_jj = Q_jj, then for the blocks above, i = j-1 .. 0,
-// V_ij = -Q_ii sum_{k=i+1}^{j} U_ik V_kj. Same layout as strip_winv_kernel.
+// V_ij = -Q_ii sum_{k=i+1}^{j} U_ik V_kj. Same layout as strip_winv_body.
 template <class C2>
-__device__ __forceinline__ void panel_vinv_body(const BatchT<C2>& b, int k0) {
+__device__ __forceinline__ void panel_vinv_body(const BatchT<C2>& b, int k0, int j) {
   extern __shared__ __align__(16) unsigned char pv_sm[];
   constexpr int BB = LU_NB * LU_NB;
   C2* Vc = reinterpret_cast<C2*>(pv_sm);   // [SW_BLK][BB] column block j of V
@@ -691,34 +977,46 @@ __device__ __forceinline__ void panel_vinv_body(const BatchT<C2>& b, int k0) {
   const C2* A = b.sys(blockIdx.z);
   const C2* Q = b.pinv + (long long)blockIdx.z * PINV_SCRATCH + PINV_Q_OFF;
   C2* V = b.pinv + (long long)blockIdx.z * PINV_SCRATCH + PINV_V_OFF;
-  const int r = threadIdx.x % LU_NB, c = threadIdx.x / LU_NB, e = r + LU_NB * c;
-  for (int k = 1; k < SW_BLK; ++k)
+  const int r = threadIdx.x % LU_NB, cg = threadIdx.x / LU_NB;
+  for (int k = 1; k <= j; ++k)
     for (int i = 0; i < k; ++i)
-      Us[((k * (k - 1)) / 2 + i) * BB + e] = A[(k0 + i * LU_NB + r) + (long long)n * (k0 + k * LU_NB + c)];
-  for (int i = 0; i < SW_BLK; ++i) Qs[i * BB + e] = Q[i * BB + e];
-  for (int j = 0; j < SW_BLK; ++j) {
-    __syncthreads();
-    Vc[j * BB + e] = Qs[j * BB + e];
-    for (int i = j - 1; i >= 0; --i) {
-      __syncthreads();   // V_kj for k > i are in shared memory
-      C2 acc = mkc<C2>(0., 0.);
-      for (int k = i + 1; k <= j; ++k) {
-        const C2* U = Us + ((k * (k - 1)) / 2 + i) * BB + r;
-        const C2* Vk = Vc + k * BB + LU_NB * c;
-#pragma unroll 8
-        for (int m = 0; m < LU_NB; ++m) cmac(acc, U[LU_NB * m], Vk[m]);
+#pragma unroll
+      for (int q = 0; q < PI_PER; ++q) {
+        const int c = cg + PI_CG * q;
+        Us[((k * (k - 1)) / 2 + i) * BB + r + LU_NB * c] = A[(k0 + i * LU_NB + r) + (long long)n * (k0 + k * LU_NB + c)];
       }
-      S[e] = acc;
-      __syncthreads();
-      const C2* Qi = Qs + i * BB + r;
-      C2 w = mkc<C2>(0., 0.);
-#pragma unroll 8
-      for (int m = 0; m < LU_NB; ++m) cmac(w, Qi[LU_NB * m], S[m + LU_NB * c]);
-      Vc[i * BB + e] = mkc<C2>(-w.x, -w.y);
+  for (int i = 0; i <= j; ++i)
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) {
+      const int e = r + LU_NB * (cg + PI_CG * q);
+      Qs[i * BB + e] = Q[i * BB + e];
     }
-    __syncthreads();
-    for (int i = 0; i <= j; ++i) V[(i * LU_NB + r) + LU_OUTER * (j * LU_NB + c)] = Vc[i * BB + e];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PI_PER; ++q) {
+    const int e = r + LU_NB * (cg + PI_CG * q);
+    Vc[j * BB + e] = Qs[j * BB + e];
   }
+  for (int i = j - 1; i >= 0; --i) {
+    __syncthreads();   // V_kj for k > i are in shared memory
+    C2 acc[PI_PER], v[PI_PER];
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) acc[q] = v[q] = mkc<C2>(0., 0.);
+    for (int k = i + 1; k <= j; ++k) blk_mac(acc, Us + ((k * (k - 1)) / 2 + i) * BB, Vc + k * BB, r, cg);
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) S[r + LU_NB * (cg + PI_CG * q)] = acc[q];
+    __syncthreads();
+    blk_mac(v, Qs + i * BB, S, r, cg);
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) Vc[i * BB + r + LU_NB * (cg + PI_CG * q)] = mkc<C2>(-v[q].x, -v[q].y);
+  }
+  __syncthreads();
+  for (int i = 0; i <= j; ++i)
+#pragma unroll
+    for (int q = 0; q < PI_PER; ++q) {
+      const int c = cg + PI_CG * q;
+      V[(i * LU_NB + r) + LU_OUTER * (j * LU_NB + c)] = Vc[i * BB + r + LU_NB * c];
+    }
 }
 
 // L21 = A21 V for the rows below the panel: CTA = one system and PL_R rows
@@ -794,18 +1092,19 @@ __device__ __forceinline__ void panel_l21_body(const BatchT<C2>& b, int k0, int 
 }
 
 template <class C2>
-__global__ void __launch_bounds__(LU_NB * LU_NB) strip_winv_kernel(BatchT<C2> b, int k0) {
-  strip_winv_body(b, k0);
+__global__ void __launch_bounds__(PI_THREADS) strip_winv_kernel(BatchT<C2> b, int k0) {
+  strip_winv_body(b, k0, blockIdx.x);
 }
 template <class C2>
 __global__ void __launch_bounds__(128) strip_gemm_kernel(BatchT<C2> b, int k0) {
   strip_gemm_body(b, k0, blockIdx.x);
 }
-// both triangle inverses of the panel's diagonal block: blockIdx.x 0 W, 1 V
+// both triangle inverses of the panel's diagonal block, a column block per
+// CTA: blockIdx.x < SW_BLK W, the others V
 template <class C2>
-__global__ void __launch_bounds__(LU_NB * LU_NB) panel_inv_kernel(BatchT<C2> b, int k0) {
-  if (blockIdx.x == 0) strip_winv_body(b, k0);
-  else panel_vinv_body(b, k0);
+__global__ void __launch_bounds__(PI_THREADS) panel_inv_kernel(BatchT<C2> b, int k0) {
+  if (blockIdx.x < SW_BLK) strip_winv_body(b, k0, blockIdx.x);
+  else panel_vinv_body(b, k0, blockIdx.x - SW_BLK);
 }
 // both block products of the panel: blockIdx.y 0 L21 = A21 V (row chunks),
 // 1 U12 = W A12 (column chunks)
@@ -960,7 +1259,7 @@ inline void lu_two_level(BatchT<C2> b, int nsys, int* status, cudaStream_t main,
         panel_block_kernel<C2><<<dim3(1, 1, ns), 1024, panel_block_smem<C2>(), st>>>(bg, k0, status);
         ++launches;
         if (kend >= ng) continue;
-        panel_inv_kernel<C2><<<dim3(2, 1, ns), LU_NB * LU_NB, strip_winv_smem<C2>(), st>>>(bg, k0);
+        panel_inv_kernel<C2><<<dim3(2 * SW_BLK, 1, ns), PI_THREADS, strip_winv_smem<C2>(), st>>>(bg, k0);
         ++launches;
         if (!outer_products) {   // else outer() forms L21 and U12 (on the tensor cores) before its update
           const int nx = std::max((ng - kend + PL_R - 1) / PL_R, (ng - kend + ST_C - 1) / ST_C);
@@ -1002,7 +1301,7 @@ inline void lu_two_level(BatchT<C2> b, int nsys, int* status, cudaStream_t main,
         const cudaStream_t st = L.st[g];
         lu_diag_kernel<C2><<<dim3(1, 1, ns), LU_DIAG_THREADS, 0, st>>>(bg, k, status);
         ++launches;
-        lu_panel_kernel<C2><<<dim3(std::max(1, nrb + ncb_used), 1, ns), LU_RB, 0, st>>>(bg, k, ucol);
+        lu_panel_kernel<C2><<<dim3(std::max(1, nrb + ncb_used), 1, ns), LU_PT, 0, st>>>(bg, k, ucol);
         ++launches;
         if (k + nb < kend) {
           zgemm_update<C2>(bg, k, nb, Rect{k + nb, ng, k + nb, kend}, ns, st);
@@ -1035,7 +1334,7 @@ inline void lu_two_level(BatchT<C2> b, int nsys, int* status, cudaStream_t main,
         });
         const dim3 sgrid((ng - kend + ST_C - 1) / ST_C, 1, ns);
         if (strip_as_product()) {
-          strip_winv_kernel<C2><<<dim3(1, 1, ns), LU_NB * LU_NB, strip_winv_smem<C2>(), st>>>(bg, k0);
+          strip_winv_kernel<C2><<<dim3(SW_BLK, 1, ns), PI_THREADS, strip_winv_smem<C2>(), st>>>(bg, k0);
           strip_gemm_kernel<C2><<<sgrid, 128, strip_gemm_smem<C2>(), st>>>(bg, k0);
           launches += 2;
         } else {

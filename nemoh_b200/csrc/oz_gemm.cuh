@@ -56,10 +56,10 @@ constexpr int OZ_SMEM = OZ_SLOTS * OZ_SLOT + 256;
 constexpr int OZ_EMIN = -250;                    // smallest scale exponent (rows and columns below it are round-off)
 // Trailing entries of a batch (over its systems) from which an update takes this
 // path; below it the FP64 pipe's one launch is as fast as the images and the
-// update, which then cover few SMs. LU in ms, FP64 pipe against this path:
-// 20 systems of 300 panels (0.6 M entries) 1.25 / 1.30, 10 of 588 (2.1 M) 2.42 /
-// 2.47, 2 of 1,430 (3.4 M) 5.44 / 5.51, 1 of 2,380 (5.1 M) 9.55 / 9.34, 20 of 588
-// (4.2 M) 2.81 / 2.75, 4 of 1,430 (6.8 M) 6.27 / 6.05, 20 of 2,380 45.0 / 28.8.
+// update, which then cover few SMs. LU in ms, FP64 pipe against this path: 10
+// systems of 420 panels (0.9 M entries) 0.74 / 0.82, 4 of 894 (2.3 M) 1.37 / 1.45,
+// 2 of 1,430 (3.4 M) 2.23 / 2.26, 20 of 588 (4.2 M) 1.47 / 1.47, 1 of 2,380 (5.1 M)
+// 4.19 / 3.99, 4 of 1,430 (6.8 M) 3.06 / 2.80, 20 of 2,380 (101 M) 37.8 / 22.2.
 constexpr double OZ_MIN_ENTRIES = 4.2e6;
 // slices in the order a chunk needs them: the first diagonal (i + j = 7) starts
 // from the middle, slice 0 is not in it
