@@ -545,11 +545,11 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
   Batch b = dbatch(c, sh);
   const int N = sh.n;
   const bool images = fp64_images(c, nsys, N);
-  // Panel pairs are merged: after an even panel only the next panel's columns
-  // and rows are updated, the rest of the trailing matrix takes both panels'
-  // products in the next panel's update, so its bulk is read and written once
-  // per pair. deferred: the groups (by their first system) whose last panel's
-  // bulk is still to come.
+  // Panel pairs are merged where the update fills the device: after the first
+  // panel only the next panel's columns and rows are updated, the rest of the
+  // trailing matrix takes both panels' products in the next panel's update, so
+  // its bulk is read and written once per pair. deferred: the groups (by their
+  // first system) whose last panel's bulk is still to come.
   std::map<int, bool> deferred;
   static std::atomic<unsigned long long> attr{0};
   once_per_device(attr, [] {
@@ -572,14 +572,11 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
         int* status = c->d_status.as<int>();
         oz_prep(cur, st, bg, k0, ns, sg, c->launches);
         if (late) {
-          oz_apply(cur, oz_set(c->oz, set ^ 1, s0), st, bg, k0, ns, sg, c->launches, status, TcTiles());
+          oz_apply(cur, oz_set(c->oz, set ^ 1, s0), st, bg, k0, ns, sg, c->launches, status, false);
           late = false;
-        } else if (kend + LU_OUTER < bg.n) {
-          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, TcTiles{0, -1, 0, 1});
-          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, TcTiles{0, 1, 1, -1});
-          late = true;
         } else {
-          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, TcTiles());
+          late = kend + LU_OUTER < bg.n && oz_tiles((int)rest, nsys) >= OZ_MERGE_TILES;
+          oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, late);
         }
       },
       &c->lanes, sh.rg.host_ord);

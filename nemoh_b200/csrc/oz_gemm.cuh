@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <utility>
 
 #include "linalg.cuh"
 #include "tc_gemm.cuh"
@@ -47,28 +48,129 @@ constexpr int OZ_PLANE = OZ_N * OZ_KC;           // 4 KB: one plane of a B slice
 constexpr int OZ_B = 3 * OZ_PLANE;               // 12 KB: one slice of a B chunk
 constexpr int OZ_ASBO = 2 * OZ_KC * 8;           // bytes between 8-row groups of an A slice
 constexpr int OZ_BSBO = OZ_KC * 8;               // and of a B plane
-constexpr int OZ_SLOT = OZ_A + OZ_B;             // 28 KB: slice i of both operands
-constexpr int OZ_SLOTS = 8;                      // the seven slices of a chunk and one ahead
+constexpr int OZ_SLOT = OZ_A + OZ_B;             // 28 KB: one slice of both operands
+constexpr int OZ_SLOTS = 8;
 constexpr int OZ_ACC = 4;                        // accumulators of 128 tensor-memory columns
-constexpr int OZ_THREADS = 320;                  // producer, MMA issuer, eight epilogue warps
-constexpr int OZ_EPI = 256;
-constexpr int OZ_SMEM = OZ_SLOTS * OZ_SLOT + 256;
+constexpr int OZ_EPI_WARPS = 16;
+constexpr int OZ_THREADS = 128 + 32 * OZ_EPI_WARPS;   // producer, two MMA issuers, an idle warp; the epilogue's
+constexpr int OZ_EC = OZ_N / (OZ_EPI_WARPS / 4);   // complex columns per epilogue thread
+constexpr int OZ_BATCH = 2;                        // of them loaded at once
+constexpr int OZ_SMEM = OZ_SLOTS * OZ_SLOT + 256 + 2 * 2 * OZ_N * (int)sizeof(double);
 constexpr int OZ_EMIN = -250;                    // smallest scale exponent (rows and columns below it are round-off)
 // Trailing entries of a batch (over its systems) from which an update takes this
 // path; below it the FP64 pipe's one launch is as fast as the images and the
 // update, which then cover few SMs. LU in ms, FP64 pipe against this path: 10
-// systems of 420 panels (0.9 M entries) 0.74 / 0.82, 4 of 894 (2.3 M) 1.37 / 1.45,
-// 2 of 1,430 (3.4 M) 2.23 / 2.26, 20 of 588 (4.2 M) 1.47 / 1.47, 1 of 2,380 (5.1 M)
-// 4.19 / 3.99, 4 of 1,430 (6.8 M) 3.06 / 2.80, 20 of 2,380 (101 M) 37.8 / 22.2.
-constexpr double OZ_MIN_ENTRIES = 4.2e6;
-// slices in the order a chunk needs them: the first diagonal (i + j = 7) starts
-// from the middle, slice 0 is not in it
-constexpr unsigned OZ_ORDER = 0x0162543u;        // nibble p: the p-th slice loaded
+// systems of 420 panels (0.9 M entries) 0.71 / 0.71, 4 of 588 (0.8 M) 0.94 / 0.95,
+// 2 of 894 (1.2 M) 1.08 / 1.08, 4 of 894 (2.3 M) 1.32 / 1.22, 2 of 1,430 (3.4 M)
+// 2.24 / 1.99, 20 of 588 (4.2 M) 1.44 / 1.25, 1 of 2,380 (5.1 M) 4.21 / 3.37, 20 of
+// 2,380 (101 M) 37.0 / 17.2.
+constexpr double OZ_MIN_ENTRIES = 1.5e6;
+// Tiles of a full update from which panel pairs are merged (four per SM): the
+// merged form reads and writes the trailing block once per pair, the corner
+// update it needs is a launch of one tile's latency more. LU in ms, never merged /
+// merged from 148 tiles / from 600: 20 systems of 420 0.77 / 0.81 / 0.78, 10 of 894
+// 1.51 / 1.52 / 1.48, 1 of 2,380 3.41 / 3.40 / 3.37, 20 of 2,380 18.7 / 18.8 / 17.2.
+constexpr long long OZ_MERGE_TILES = 600;
+
+// The schedule of a tile. Its 68 slice products run in four phases: diagonals 7 ..
+// 4 of both chunks into the four accumulators, then diagonals 0 .. 3 of both
+// chunks (slices 0 .. 3, loaded again), so that an accumulator is drained once per
+// phase pair and not once per chunk: the FP64 pipe and the tensor pipe do not run
+// at the same time (measured: 384 k cycles of DFMA and 410 k of MMA take 833 k
+// together), and every drained value costs FP64 work.
+// Each step is one slice product (A slice i, B slice j) of a phase. The order lets
+// slices retire early and lets the accumulators finish in pairs, (0, 1) before
+// (2, 3), which are drained and free again before the next phase pair meets them;
+// slices of one phase lie in other slots than those of the next where the same
+// slot would free up too late. A load is (slice, slot).
+struct OzStep {
+  signed char i, j;      // slices of A and B
+  signed char slot_i, slot_j;
+  signed char acc;       // accumulator
+  signed char first;     // first product of its accumulator
+  short need;            // slots to wait for, as a bit mask
+  short retire;          // slots no later step of the phase reads, as a bit mask
+  signed char full;      // accumulators finished, as a bit mask
+};
+template <int N>
+struct OzPhase {
+  OzStep s[N];
+  int count;   // steps in use
+};
+// The steps of one issuer (accumulators `mine`, a bit mask) of a phase.
+// slots[i]: slot of slice i (nsl slices); pairs: (i, j) in order; low: diagonals 0
+// .. 3 (accumulator i + j), else 7 .. 4 (accumulator 7 - i - j); begin / end: the
+// first / last chunk of the phase pair. Both issuers wait for and release every
+// slot of the phase (a slot's barrier counts two releases), one that it does not
+// read with its last step.
+template <int N>
+constexpr OzPhase<N> oz_phase(const int (&pairs)[N][2], const int (&slots)[OZ_S], int nsl, bool low, bool begin,
+                              bool end, int mine) {
+  OzPhase<N> p{};
+  int all = 0;
+  for (int i = 0; i < nsl; ++i) all |= 1 << slots[i];
+  int seen = 0, used = 0;
+  for (int k = 0; k < N; ++k) {
+    const int i = pairs[k][0], j = pairs[k][1], acc = low ? i + j : 7 - i - j;
+    if (!((mine >> acc) & 1)) continue;
+    OzStep& t = p.s[p.count++];
+    t.i = (signed char)i;
+    t.j = (signed char)j;
+    t.slot_i = (signed char)slots[i];
+    t.slot_j = (signed char)slots[j];
+    t.acc = (signed char)acc;
+    t.first = begin && !((used >> acc) & 1);
+    used |= 1 << acc;
+    int m = (1 << slots[i]) | (1 << slots[j]);
+    int later = 0, open = 0;
+    for (int q = k + 1; q < N; ++q) {
+      const int a = low ? pairs[q][0] + pairs[q][1] : 7 - pairs[q][0] - pairs[q][1];
+      if (!((mine >> a) & 1)) continue;
+      later |= (1 << slots[pairs[q][0]]) | (1 << slots[pairs[q][1]]);
+      open |= 1 << a;
+    }
+    if (later == 0) m |= all & ~(seen | m);   // the last step
+    t.need = (short)(m & ~seen);
+    seen |= m;
+    t.retire = (short)(m & ~later);
+    t.full = (signed char)(end && !((open >> acc) & 1) ? 1 << acc : 0);
+  }
+  return p;
+}
+constexpr int OZ_P0[24][2] = {{1, 6}, {6, 1}, {1, 5}, {5, 1}, {1, 4}, {4, 1}, {0, 6}, {6, 0},
+                              {0, 5}, {5, 0}, {0, 4}, {4, 0}, {2, 5}, {5, 2}, {2, 4}, {4, 2},
+                              {2, 2}, {3, 4}, {4, 3}, {3, 3}, {2, 3}, {3, 2}, {1, 3}, {3, 1}};
+constexpr int OZ_P1[24][2] = {{1, 6}, {6, 1}, {1, 5}, {5, 1}, {0, 6}, {6, 0}, {2, 5}, {5, 2},
+                              {2, 4}, {4, 2}, {3, 4}, {4, 3}, {3, 3}, {0, 5}, {5, 0}, {1, 4},
+                              {4, 1}, {2, 3}, {3, 2}, {0, 4}, {4, 0}, {1, 3}, {3, 1}, {2, 2}};
+constexpr int OZ_P2[10][2] = {{0, 0}, {0, 1}, {1, 0}, {1, 1}, {0, 2}, {2, 0}, {1, 2}, {2, 1}, {0, 3}, {3, 0}};
+constexpr int OZ_P3[10][2] = {{0, 0}, {0, 1}, {1, 0}, {0, 2}, {2, 0}, {1, 1}, {1, 2}, {2, 1}, {0, 3}, {3, 0}};
+constexpr int OZ_L0[OZ_S] = {0, 1, 2, 3, 4, 5, 6}, OZ_L1[OZ_S] = {0, 7, 2, 3, 4, 5, 6},
+              OZ_L2[OZ_S] = {6, 1, 5, 4, 0, 0, 0}, OZ_L3[OZ_S] = {0, 7, 2, 3, 0, 0, 0};
+// Two warps issue, each with two of the accumulators: an MMA is handed over only
+// about when the one before it starts (measured: a pause of 200 cycles after every
+// four MMAs costs 219), so one issuer's waits and releases would leave the tensor
+// pipe idle; the other's MMAs fill them.
+constexpr int OZ_WHO0 = (1 << 0) | (1 << 3), OZ_WHO1 = (1 << 1) | (1 << 2);
+template <int WHO>
+struct OzPlan {
+  static constexpr OzPhase<24> p0 = oz_phase(OZ_P0, OZ_L0, 7, false, true, false, WHO);
+  static constexpr OzPhase<24> p1 = oz_phase(OZ_P1, OZ_L1, 7, false, false, true, WHO);
+  static constexpr OzPhase<10> p2 = oz_phase(OZ_P2, OZ_L2, 4, true, true, false, WHO);
+  static constexpr OzPhase<10> p3 = oz_phase(OZ_P3, OZ_L3, 4, true, false, true, WHO);
+};
+// the loads of a tile in the order their slots free up: nibbles slice, slot
+constexpr int OZ_LOADS = 22;
+constexpr signed char OZ_LOAD[OZ_LOADS][3] = {   // slice, slot, chunk
+    {1, 1, 0}, {6, 6, 0}, {5, 5, 0}, {4, 4, 0}, {0, 0, 0}, {2, 2, 0}, {3, 3, 0},
+    {1, 7, 1}, {6, 6, 1}, {0, 0, 1}, {5, 5, 1}, {4, 4, 1}, {2, 2, 1}, {3, 3, 1},
+    {1, 1, 0}, {0, 6, 0}, {2, 5, 0}, {3, 4, 0},
+    {0, 0, 1}, {1, 7, 1}, {2, 2, 1}, {3, 3, 1}};
 
 // Operand images and scales of two panels (the update of one panel may be
-// merged into the next one's): per system and set, ceil(n / 128) row tiles and
-// 2 ceil(n / 128) column tiles of OZ_NCH chunks of OZ_S slices; scales one per
-// row, then one per column.
+// merged into the next one's): per set and system ceil(n / 128) row tiles and 2
+// ceil(n / 128) column tiles of OZ_NCH chunks of OZ_S slices; scales one per row,
+// then one per column.
 struct OzWork {
   unsigned char* a = nullptr;
   unsigned char* b = nullptr;
@@ -102,8 +204,8 @@ inline size_t oz_bytes_per_system(size_t n) {
   return t * (OZ_NCH * OZ_S * (size_t)(OZ_A + 2 * OZ_B) + 2 * OZ_M * sizeof(double));
 }
 
-// The images of one panel as the kernels take them (bases of the launch's
-// first system): strides are per system.
+// The images as the kernels take them (bases of the launch's first system):
+// strides are per system.
 struct OzSet {
   unsigned char* a = nullptr;
   unsigned char* b = nullptr;
@@ -270,65 +372,219 @@ __device__ __forceinline__ void oz_mma(uint32_t tmem, uint64_t da, uint64_t db, 
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(addr));
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t* a, uint32_t* b) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) asm volatile("" : "+r"(a[i]), "+r"(b[i]));   // the values are there only now
 }
 
-// The update of a rectangle of tiles (row tiles [ti0, ti0 + nti), column tiles
-// [tj0, tj0 + ntc) of 128 x 64 complex) of every system, one persistent CTA per
-// SM walking tile t, t + grid, ...:
-//   warp 0 (one thread)  loads slice i of A and B (28 KB) into one of eight
-//                        slots; the slots free up as the diagonals go down;
-//   warp 1 (one thread)  issues the MMAs of a chunk diagonal by diagonal, i + j
-//                        = 7 first, then 6 .. 0 (slice s is done with diagonal
-//                        s, so its slot takes the next chunk's slice while the
-//                        diagonals below still run), each into one of four
-//                        128-column accumulators;
-//   warps 2-9            add a finished diagonal to the tile's FP64 sums (64 per
-//                        thread, in registers; warp w the TMEM lanes 32 (w % 4)
-//                        .. and half (w - 2) / 4 of the columns) and, after the
-//                        last chunk, subtract the scaled sums from A22.
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0;
+}
+
+// Step K of a phase: waits for the slices and the accumulator it meets first,
+// issues its four MMAs, and releases the slots and accumulators it is the last of.
+// sync.full(slot) / sync.empty(acc) wait, uniformly over the warp.
+template <const auto& PH, int K, class Sync>
+__device__ __forceinline__ bool oz_step(uint32_t tmem, uint64_t da, uint64_t db, bool issue, uint32_t empty0,
+                                        uint32_t accf0, Sync& sync) {
+  constexpr OzStep t = PH.s[K];
+  if (t.first && !sync.empty(t.acc)) return false;
+#pragma unroll
+  for (int q = 0; q < OZ_SLOTS; ++q)
+    if ((t.need >> q) & 1)
+      if (!sync.full(q)) return false;
+  if (issue) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)   // Ar against (Br, Bi), then Ai against (-Bi, Br)
+      oz_mma(tmem + t.acc * 2 * OZ_N, da + (uint64_t)((t.slot_i * OZ_SLOT + kk * 256) >> 4),
+             db + (uint64_t)((t.slot_j * OZ_SLOT + (kk < 2 ? OZ_PLANE : 0) + (kk & 1) * 256) >> 4),
+             (kk > 0 || !t.first) ? 1u : 0u);
+    if (t.full)
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(accf0 +
+                                                                                                       8 * t.acc)
+                   : "memory");
+#pragma unroll
+    for (int q = 0; q < OZ_SLOTS; ++q)
+      if ((t.retire >> q) & 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty0 + 8 * q)
+                     : "memory");
+  }
+  __syncwarp();
+  return true;
+}
+template <const auto& PH, class Sync, int... K>
+__device__ __forceinline__ bool oz_steps(std::integer_sequence<int, K...>, uint32_t tmem, uint64_t da, uint64_t db,
+                                         bool issue, uint32_t empty0, uint32_t accf0, Sync& sync) {
+  return (oz_step<PH, K>(tmem, da, db, issue, empty0, accf0, sync) && ...);
+}
+template <const auto& PH, class Sync>
+__device__ __forceinline__ bool oz_run(uint32_t tmem, uint64_t da, uint64_t db, bool issue, uint32_t empty0,
+                                       uint32_t accf0, Sync& sync) {
+  return oz_steps<PH>(std::make_integer_sequence<int, PH.count>{}, tmem, da, db, issue, empty0, accf0, sync);
+}
+
+// The waits of the MMA issuer (by every lane of its warp).
+struct OzSync {
+  uint32_t full0, acce0;
+  uint32_t fph = 0;    // parity of the next full wait per slot
+  uint32_t aph = 0;    // parity of the next empty wait per accumulator
+  uint32_t used = 0;   // accumulators used before
+  __device__ __forceinline__ bool full(int q) {
+    const bool got = mbar_wait_suspend(full0 + 8 * q, (fph >> q) & 1);
+    fph ^= 1u << q;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return __all_sync(0xffffffffu, got) != 0;
+  }
+  __device__ __forceinline__ bool empty(int a) {
+    bool got = true;
+    if ((used >> a) & 1) {
+      got = mbar_wait_suspend(acce0 + 8 * a, (aph >> a) & 1);
+      aph ^= 1u << a;
+    }
+    used |= 1u << a;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return __all_sync(0xffffffffu, got) != 0;
+  }
+};
+
+// Load L of a tile's schedule: waits until its slot is free and copies a slice of
+// A and B into it. used: slots loaded before; eph, fph: parity of the next empty
+// wait and of the last load per slot.
+template <int L>
+__device__ __forceinline__ bool oz_load(const unsigned char* ga, const unsigned char* gb, uint32_t s0, uint32_t full0,
+                                        uint32_t empty0, uint32_t& used, uint32_t& eph, uint32_t& fph) {
+  constexpr int i = OZ_LOAD[L][0], q = OZ_LOAD[L][1], c = OZ_LOAD[L][2];
+  if ((used >> q) & 1) {
+    if (!mbar_wait_suspend(empty0 + 8 * q, (eph >> q) & 1)) return false;
+    eph ^= 1u << q;
+    fph ^= 1u << q;
+  }
+  used |= 1u << q;
+  const uint32_t dst = s0 + q * OZ_SLOT, bar = full0 + 8 * q;
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(OZ_SLOT) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(ga + (c * OZ_S + i) * OZ_A), "r"(OZ_A), "r"(bar)
+               : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst +
+                                                                                                             OZ_A),
+               "l"(gb + (c * OZ_S + i) * OZ_B), "r"(OZ_B), "r"(bar)
+               : "memory");
+  return true;
+}
+template <int... L>
+__device__ __forceinline__ bool oz_load_tile(std::integer_sequence<int, L...>, const unsigned char* ga,
+                                             const unsigned char* gb, uint32_t s0, uint32_t full0, uint32_t empty0,
+                                             uint32_t& used, uint32_t& eph, uint32_t& fph) {
+  return (oz_load<L>(ga, gb, s0, full0, empty0, used, eph, fph) && ...);
+}
+
+// a thread's row of the tile: C -= rs cc (ar + i ai), OZ_BATCH columns at a time
+__device__ __forceinline__ void oz_subtract(double2* C, int n, int ncol, double rs, const double* cc, const double* ar,
+                                            const double* ai) {
+#pragma unroll
+  for (int q = 0; q < OZ_EC; q += OZ_BATCH) {
+    double2 v[OZ_BATCH];
+    double2* p = C;
+#pragma unroll
+    for (int j = 0; j < OZ_BATCH; ++j, p += n)
+      if (q + j < ncol) v[j] = *p;
+#pragma unroll
+    for (int j = 0; j < OZ_BATCH; ++j, C += n)
+      if (q + j < ncol) {
+        const double f = -rs * cc[q + j];
+        v[j].x = fma(ar[q + j], f, v[j].x);
+        v[j].y = fma(ai[q + j], f, v[j].y);
+        *C = v[j];
+      }
+  }
+}
+
+// The update by tiles of 128 x 64 complex (nti row tiles, ntc column tiles) of
+// every system, one persistent CTA per SM walking tile t, t + grid, ...:
+//   warp 0 (one thread)  loads slices of A and B (28 KB) into the slots, in OZ_LOAD's order;
+//   warps 1 and 2        issue the MMAs of their accumulators: the whole warp walks
+//                        the phases, so that every address is warp-uniform, and one
+//                        lane issues; the steps are written out (looked up step by
+//                        step they took longer than their MMAs);
+//   warps 4-19           add a finished pair of diagonals to the tile's FP64 sums
+//                        (32 per thread, in registers; warp w the TMEM lanes 32 (w %
+//                        4) .. and quarter (w - 4) / 4 of the columns) and, at the
+//                        end, subtract the scaled sums from A22, while the next
+//                        tile's first products run.
 // prev.a: the images of the previous panel, whose update of these tiles was
-// deferred: its chunks run first and its sums are rescaled (exactly) to this
-// panel's scales. Every wait is bounded; a role that times out raises the
-// status and flags the others, and each waits (bounded) for its own copies and
-// MMAs before the CTA frees its tensor memory.
+// deferred: its products run first and its sums are rescaled (exactly) to this
+// panel's scales. corner: the tiles of the next panel's columns and rows only.
+// Every wait is bounded; a role that times out raises the status and flags the
+// others, and each waits (bounded) for its own copies and MMAs before the CTA
+// frees its tensor memory.
+// What bounds it: the tensor pipe at 64 cycles an MMA (an N = 128 MMA reads its
+// operands from shared memory at the port's 128 B a cycle), the FP64 and integer
+// work of the drains, which takes tensor cycles, and the read-modify-write of A22,
+// 256 KB per tile. Two systems of 2,252 trailing rows: 193 us per panel (1,296
+// tiles, 17,400 cycles of MMAs each; 113 us without drains and A22), 286 us for a
+// merged pair; a first form that drained every 64 complex k took 256 and 420 us,
+// the FP64 pipe 830 us per panel.
 __global__ void __launch_bounds__(OZ_THREADS, 1)
-    oz_update_kernel(Batch b, int k0, OzSet cur, OzSet prev, OzStride st, int nsys, int* status, int ti0, int nti,
-                     int tj0, int ntc) {
+    oz_update_kernel(Batch b, int k0, OzSet cur, OzSet prev, OzStride st, int nsys, int* status, int nti, int ntc,
+                     int corner) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OZ_SLOTS * OZ_SLOT);
   // full[8], empty[8], acc_full[4], acc_empty[4], drain; then the TMEM address
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * OZ_SLOTS + 2 * OZ_ACC + 1);
+  // a tile's column scales and, in a merged update, the ratios of the deferred
+  // panel's to them; two tiles' worth
+  double(*s_col)[2][OZ_N] = reinterpret_cast<double(*)[2][OZ_N]>(smem + OZ_SLOTS * OZ_SLOT + 256);
   __shared__ volatile int s_err;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[OZ_SLOTS]);
   const uint32_t accf0 = smem_u32(&bars[2 * OZ_SLOTS]), acce0 = smem_u32(&bars[2 * OZ_SLOTS + OZ_ACC]);
   const uint32_t drain = smem_u32(&bars[2 * OZ_SLOTS + 2 * OZ_ACC]);
   const int r1 = k0 + LU_OUTER;
-  const long long total = (long long)nti * ntc * nsys;
-  const int nch = prev.a ? 2 * OZ_NCH : OZ_NCH;
+  // corner: only the first 128 columns (every row) and the first 128 rows
+  constexpr int CW = LU_OUTER / OZ_N;   // column tiles of a panel's width
+  const int per = corner ? CW * nti + max(0, ntc - CW) : nti * ntc;
+  const long long total = (long long)per * nsys;
+  const int parts = prev.a ? 2 : 1;
   auto tile = [&](long long t, int& z, int& trow, int& tcol) {
-    z = (int)(t / ((long long)nti * ntc));
-    const int rem = (int)(t % ((long long)nti * ntc));
-    trow = ti0 + rem / ntc;
-    tcol = tj0 + rem % ntc;
+    z = (int)(t / per);
+    const int rem = (int)(t % per);
+    if (!corner) {
+      trow = rem / ntc;
+      tcol = rem % ntc;
+    } else if (rem < CW * nti) {
+      trow = rem / CW;
+      tcol = rem % CW;
+    } else {
+      trow = 0;
+      tcol = rem - CW * nti + CW;
+    }
     const int rest = b.order(z) - r1;
     return rest > 0 && trow * OZ_M < rest && tcol * OZ_N < rest;
   };
   if (threadIdx.x == 0) {
     s_err = 0;
-    for (int i = 0; i < 2 * OZ_SLOTS; ++i)
+    for (int i = 0; i < OZ_SLOTS; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(empty0 + 8 * i));   // both issuers
+    }
     for (int i = 0; i < OZ_ACC; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(accf0 + 8 * i));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acce0 + 8 * i), "r"(OZ_EPI));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(acce0 + 8 * i), "r"(OZ_EPI_WARPS));
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(drain));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(drain));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -344,197 +600,139 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     atomicCAS(status, 0, ST_TC_TIMEOUT);
     s_err = 1;
   };
-  // The slot of the p-th loaded slice of a chunk, the same sequence in the
-  // producer and the issuer: first the spare slot, then the slots of the
-  // previous chunk's slices 6, 5, .. 1 as their diagonals end; the slot of
-  // slice 0 becomes the spare. `map` holds slice i's slot in nibble i, the
-  // spare in nibble 7.
-  auto next_map = [](uint32_t map) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int p = 0; p < OZ_S; ++p) {
-      const uint32_t slot = (map >> (4 * (7 - p))) & 0xf;   // nibble 7 (spare), then 6 .. 1
-      m |= slot << (4 * ((OZ_ORDER >> (4 * p)) & 0xf));
-    }
-    return m | ((map & 0xf) << 28);
-  };
-  constexpr uint32_t MAP0 = 0x76543210u;
 
   if (warp == 0 && lane == 0) {
     // producer
     const uint32_t s0 = smem_u32(smem);
-    uint32_t map = MAP0, used = 0, eph = 0, fph = 0;   // slots loaded so far; parities of the next empty / last full wait
+    uint32_t used = 0, eph = 0, fph = 0;   // slots loaded before; parity of the next empty wait and of the last load
     bool ok = true;
     for (long long t = blockIdx.x; t < total && ok && !s_err; t += gridDim.x) {
       int z, trow, tcol;
       if (!tile(t, z, trow, tcol)) continue;
-      for (int c = 0; c < nch && ok; ++c) {
+      for (int part = 0; part < parts && ok; ++part) {
         // the previous panel's trailing block starts 128 rows and columns earlier
-        const bool pv = prev.a && c < OZ_NCH;
-        const OzSet& s = pv ? prev : cur;
-        const unsigned char* ga = s.a + z * st.a + ((long long)(trow + (pv ? 1 : 0)) * OZ_NCH + c % OZ_NCH) * OZ_S * OZ_A;
-        const unsigned char* gb =
-            s.b + z * st.b + ((long long)(tcol + (pv ? OZ_M / OZ_N : 0)) * OZ_NCH + c % OZ_NCH) * OZ_S * OZ_B;
-        map = next_map(map);
-        for (int p = 0; p < OZ_S; ++p) {
-          const int i = (OZ_ORDER >> (4 * p)) & 0xf, q = (map >> (4 * i)) & 0xf;
-          if ((used >> q) & 1) {
-            if (!(ok = mbar_wait_suspend(empty0 + 8 * q, (eph >> q) & 1))) break;
-            eph ^= 1u << q;
-            fph ^= 1u << q;
-          }
-          used |= 1u << q;
-          const uint32_t dst = s0 + q * OZ_SLOT, bar = full0 + 8 * q;
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(OZ_SLOT) : "memory");
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           dst),
-                       "l"(ga + i * OZ_A), "r"(OZ_A), "r"(bar)
-                       : "memory");
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           dst + OZ_A),
-                       "l"(gb + i * OZ_B), "r"(OZ_B), "r"(bar)
-                       : "memory");
-        }
+        const bool pv = part + 1 < parts;
+        const unsigned char* ga = (pv ? prev.a : cur.a) + z * st.a + (long long)(trow + (pv ? 1 : 0)) * OZ_NCH * OZ_S * OZ_A;
+        const unsigned char* gb = (pv ? prev.b : cur.b) + z * st.b + (long long)(tcol + (pv ? CW : 0)) * OZ_NCH * OZ_S * OZ_B;
+        ok = oz_load_tile(std::make_integer_sequence<int, OZ_LOADS>{}, ga, gb, s0, full0, empty0, used, eph, fph);
       }
     }
     if (!ok) fail();
     // copies in flight land before the CTA can leave: the last load of each slot
     for (int q = 0; q < OZ_SLOTS; ++q)
       if ((used >> q) & 1) mbar_wait_suspend(full0 + 8 * q, (fph >> q) & 1);
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer
+  } else if (warp == 1 || warp == 2) {
     const uint32_t s0 = smem_u32(smem);
-    const uint64_t da0 = umma_desc(s0, 128, OZ_ASBO), db0 = umma_desc(s0 + OZ_A, 128, OZ_BSBO);
-    uint32_t map = MAP0, fph = 0;   // parity of the next full wait per slot
-    long long g = 0;                // diagonals issued
-    bool ok = true;
-    for (long long t = blockIdx.x; t < total && ok && !s_err; t += gridDim.x) {
-      int z, trow, tcol;
-      if (!tile(t, z, trow, tcol)) continue;
-      for (int c = 0; c < nch && ok; ++c) {
-        map = next_map(map);
-        uint32_t have = 0;   // slices of this chunk known to have landed
-        for (int s = OZ_D - 1; s >= 0 && ok; --s, ++g) {
-          const int buf = (int)(g % OZ_ACC);
-          if (g >= OZ_ACC && !(ok = mbar_wait_suspend(acce0 + 8 * buf, (uint32_t)((g / OZ_ACC - 1) & 1)))) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t tm = tmem + (uint32_t)(buf * 2 * OZ_N);
-          const int lo = max(0, s - (OZ_S - 1)), cnt = s - 2 * lo + 1;   // pairs (lo, s - lo) .. (s - lo, lo)
-          for (int m = 0; m < cnt; ++m) {
-            // from the middle outwards on the first diagonal (the order the slices arrive in)
-            const int mid = cnt / 2, i = lo + (s == OZ_D - 1 ? ((m & 1) ? mid + m / 2 : mid - 1 - m / 2) : m), j = s - i;
-            const int qa = (map >> (4 * i)) & 0xf, qb = (map >> (4 * j)) & 0xf;
-            for (int h = 0; h < 2 && ok; ++h) {
-              const int sl = h ? j : i, q = h ? qb : qa;
-              if (!((have >> sl) & 1)) {
-                if (!(ok = mbar_wait_suspend(full0 + 8 * q, (fph >> q) & 1))) break;
-                fph ^= 1u << q;
-                have |= 1u << sl;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              }
-            }
-            if (!ok) break;
-            const uint64_t da = da0 + (uint64_t)((qa * OZ_SLOT) >> 4), db = db0 + (uint64_t)((qb * OZ_SLOT) >> 4);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)   // Ar against (Br, Bi), then Ai against (-Bi, Br)
-              oz_mma(tm, da + (uint64_t)((kk * 256) >> 4), db + (uint64_t)(((kk < 2 ? OZ_PLANE : 0) + (kk & 1) * 256) >> 4),
-                     (m > 0 || kk > 0) ? 1u : 0u);
-          }
-          if (!ok) break;
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(accf0 +
-                                                                                                           8 * buf)
-                       : "memory");
-          if (s < OZ_S)   // slice s is in no diagonal below
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             empty0 + 8 * ((map >> (4 * s)) & 0xf))
-                         : "memory");
-        }
-      }
-    }
-    if (!ok) fail();
-    // every MMA issued has completed before the tensor memory is freed
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain) : "memory");
-    mbar_wait_suspend(drain, 0);
-  } else if (warp >= 2) {
-    // epilogue: thread = TMEM lane (row), 32 complex columns of the tile
-    const int lq = warp & 3, half = (warp - 2) >> 2;
-    const int row = lq * 32 + lane;
-    const uint32_t tl = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(32 * half);
-    long long g = 0;
+    const uint64_t da = umma_desc(s0, 128, OZ_ASBO), db = umma_desc(s0 + OZ_A, 128, OZ_BSBO);
+    const bool issue = elect_one();
+    OzSync sync{full0, acce0};
     bool ok = true;
     for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
       if (__shfl_sync(0xffffffffu, s_err, 0)) break;
       int z, trow, tcol;
+      if (!__shfl_sync(0xffffffffu, tile(t, z, trow, tcol), 0)) continue;
+      auto plan = [&](auto pl) {
+        using P = decltype(pl);
+        return oz_run<P::p0>(tmem, da, db, issue, empty0, accf0, sync) &&
+               oz_run<P::p1>(tmem, da, db, issue, empty0, accf0, sync) &&
+               oz_run<P::p2>(tmem, da, db, issue, empty0, accf0, sync) &&
+               oz_run<P::p3>(tmem, da, db, issue, empty0, accf0, sync);
+      };
+      for (int part = 0; part < parts && ok; ++part)
+        ok = warp == 1 ? plan(OzPlan<OZ_WHO0>{}) : plan(OzPlan<OZ_WHO1>{});
+    }
+    if (!ok && issue) fail();
+    // every MMA issued has completed before the tensor memory is freed
+    if (issue)
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain) : "memory");
+    __syncwarp();
+    mbar_wait_suspend(drain, 0);
+  } else if (warp >= 4) {
+    // epilogue: thread = TMEM lane (row), OZ_EC complex columns of the tile
+    const int lq = warp & 3, part_c = ((warp - 4) >> 2) * OZ_EC;
+    const int row = lq * 32 + lane;
+    const uint32_t tl = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)part_c;
+    bool ok = true;
+    int turn = 0;
+    // exact powers of two: their reciprocals are a subtraction of exponents
+    auto inverse = [](double x) { return __hiloint2double(0x7fe00000 - __double2hiint(x), 0); };
+    for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+      int z, trow, tcol;
       if (!tile(t, z, trow, tcol)) continue;
       const int n = b.order(z);
-      const int gr = r1 + trow * OZ_M + row, c0 = r1 + tcol * OZ_N + 32 * half;
-      const int ncol = min(32, n - c0);
+      turn ^= 1;
+      const long long zs = z * st.s;
+      if (warp < 4 + OZ_N / 32) {
+        const int j = (warp - 4) * 32 + lane;
+        const double cc = cur.cb[zs + tcol * OZ_N + j];
+        s_col[turn][0][j] = cc;
+        if (parts > 1) s_col[turn][1][j] = prev.cb[zs + tcol * OZ_N + OZ_M + j] * inverse(cc);
+      }
+      const double rs = cur.ra[zs + trow * OZ_M + row];
+      const double rr = parts > 1 ? prev.ra[zs + (trow + 1) * OZ_M + row] * inverse(rs) : 0.;
+      // every epilogue thread: the scales are there, and nobody reads the tile before last's
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * OZ_EPI_WARPS) : "memory");
+      ok = ok && !__shfl_sync(0xffffffffu, s_err, 0);
+      if (!ok) continue;   // the others still meet at the barrier
+      const int gr = r1 + trow * OZ_M + row, c0 = r1 + tcol * OZ_N + part_c;
+      const int ncol = min(OZ_EC, n - c0);
       double2* C = b.sys(z) + gr + (long long)n * c0;
       // the tile comes into L2 while its products run
       if (gr < n && (lane & 7) == 0)
         for (int j = 0; j < ncol; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (long long)n * j));
-      double ar[32], ai[32];
+      double ar[OZ_EC], ai[OZ_EC];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) ar[j] = ai[j] = 0.;
-      for (int c = 0; c < nch && ok; ++c) {
-        if (prev.a && c == OZ_NCH) {   // the deferred panel's sums in this panel's scales
-          const double* pr = prev.ra + z * st.s + (trow + 1) * OZ_M + row;
-          const double* pc = prev.cb + z * st.s + tcol * OZ_N + OZ_M + 32 * half;
-          const double* cc = cur.cb + z * st.s + tcol * OZ_N + 32 * half;
-          const double rr = *pr / cur.ra[z * st.s + trow * OZ_M + row];
+      for (int j = 0; j < OZ_EC; ++j) ar[j] = ai[j] = 0.;
+      // accumulator pairs: diagonals (7, 6), (5, 4) of the first phase pair, (0, 1), (2, 3)
+      // of the second; the lighter diagonal is the odd one
+#pragma unroll 1
+      for (int pq = 0; pq < 4 * parts && ok; ++pq) {
+        const int q = pq & 3;
+        if (pq == 4) {
+          // the deferred panel's sums in this panel's scales, exactly
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const double f = rr * (pc[j] / cc[j]);
+          for (int j = 0; j < OZ_EC; ++j) {
+            const double f = rr * s_col[turn][1][part_c + j];
             ar[j] *= f;
             ai[j] *= f;
           }
         }
-        double wt = 1.;   // weight of the diagonal: 256^(7 - s)
-        for (int s = OZ_D - 1; s >= 0; --s, ++g, wt *= 256.) {
-          const int buf = (int)(g % OZ_ACC);
-          const bool got = mbar_wait_suspend(accf0 + 8 * buf, (uint32_t)((g / OZ_ACC) & 1));
-          if (!(ok = __all_sync(0xffffffffu, got))) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t ta = tl + (uint32_t)(buf * 2 * OZ_N);
-          uint32_t v[16];
-          // INT32 -> FP64 by its bits: 2^52 + 2^31 + v, exactly
-          auto value = [](uint32_t x) { return __hiloint2double(0x43300000, (int)(x ^ 0x80000000u)) - 4503601774854144.; };
+        const int a0 = 2 * (q & 1);
+        const bool got = mbar_wait_suspend(accf0 + 8 * a0, q >> 1) && mbar_wait_suspend(accf0 + 8 * (a0 + 1), q >> 1);
+        if (!(ok = __all_sync(0xffffffffu, got))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tlo = tl + (uint32_t)((q < 2 ? a0 : a0 + 1) * 2 * OZ_N);   // diagonals 7, 5, 1, 3
+        const uint32_t thi = tl + (uint32_t)((q < 2 ? a0 + 1 : a0) * 2 * OZ_N);   // diagonals 6, 4, 0, 2
+        // weight of the lighter diagonal, 256^(7 - s): 1, 2^16, 2^48, 2^32
+        const double wt = __hiloint2double((1023 + (q < 2 ? 16 * q : 80 - 16 * q)) << 20, 0);
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {   // Re columns 0..15, 16..31, Im columns 0..15, 16..31
-            tmem_ld16(ta + (h >> 1) * OZ_N + (h & 1) * 16, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (h == 3) {   // the accumulator is read: release it
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * buf) : "memory");
+        for (int h = 0; h < 2 * OZ_EC / 8; ++h) {   // eight columns of Re, then of Im
+          constexpr int HR = OZ_EC / 8;
+          uint32_t lo[8], hi[8];
+          const uint32_t off = (uint32_t)((h / HR) * OZ_N + (h % HR) * 8);
+          tmem_ld8(tlo + off, lo);
+          tmem_ld8(thi + off, hi);
+          tmem_ld_wait(lo, hi);
+          if (h == 2 * HR - 1) {   // both accumulators are read: release them
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * a0) : "memory");
+              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * (a0 + 1)) : "memory");
             }
+          }
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              double& a = h < 2 ? ar[16 * (h & 1) + j] : ai[16 * (h & 1) + j];
-              a = fma(value(v[j]), wt, a);
-            }
+          for (int j = 0; j < 8; ++j) {
+            // v = 256 hi + lo, |v| < 2^34, as the double 2^52 + 2^51 + 2^31 + v by its bits
+            const long long bits = (long long)(int)hi[j] * 256 +
+                                   (long long)(0x4338000000000000ull | (unsigned long long)(lo[j] ^ 0x80000000u));
+            const double v = __longlong_as_double(bits) - 6755401588539392.;
+            double& a = h < HR ? ar[8 * (h % HR) + j] : ai[8 * (h % HR) + j];
+            a = fma(v, wt, a);
           }
         }
       }
-      if (!ok) break;
-      if (gr < n) {
-        const double rs = cur.ra[z * st.s + trow * OZ_M + row];
-        const double* cc = cur.cb + z * st.s + tcol * OZ_N + 32 * half;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          double2 v[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (4 * q + j < ncol) v[j] = C[(long long)n * (4 * q + j)];
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (4 * q + j < ncol) {
-              const double f = -rs * cc[4 * q + j];
-              v[j].x = fma(ar[4 * q + j], f, v[j].x);
-              v[j].y = fma(ai[4 * q + j], f, v[j].y);
-              C[(long long)n * (4 * q + j)] = v[j];
-            }
-        }
-      }
+      if (ok && gr < n) oz_subtract(C, n, ncol, rs, &s_col[turn][0][part_c], ar, ai);
     }
     if (!ok) fail();
   }
@@ -555,19 +753,19 @@ inline void oz_prep(const OzSet& s, const OzStride& st, Batch b, int k0, int nsy
   ++launches;
 }
 
-// A[r1 + 128 i0 :, r1 + 128 j0 :] of the panel's trailing block, `ni` x `nj`
-// blocks of 128 (negative: to the end), from the images in cur (and the
-// deferred panel's in prev)
+// tiles of a full update of the trailing block
+inline long long oz_tiles(int rest, int nsys) {
+  return (long long)((rest + OZ_M - 1) / OZ_M) * ((rest + OZ_N - 1) / OZ_N) * nsys;
+}
+
+// The panel's trailing block from its images (and the deferred panel's in prev);
+// corner: only what the next panel needs, its 128 columns and rows
 inline void oz_apply(const OzSet& cur, const OzSet& prev, const OzStride& st, Batch b, int k0, int nsys,
-                     cudaStream_t stream, long long& launches, int* status, TcTiles tl) {
+                     cudaStream_t stream, long long& launches, int* status, bool corner) {
   const int rest = b.n - k0 - LU_OUTER;
   if (rest <= 0) return;
-  const int nt = (rest + OZ_M - 1) / OZ_M, nc = (rest + OZ_N - 1) / OZ_N;
-  constexpr int CPB = OZ_M / OZ_N;   // column tiles per block of 128
-  const int nti = std::min(tl.nti < 0 ? nt - tl.ti0 : tl.nti, nt - tl.ti0);
-  const int tj0 = CPB * tl.tj0;
-  const int ntc = std::min(tl.ntc < 0 ? nc - tj0 : CPB * tl.ntc, nc - tj0);
-  if (nti <= 0 || ntc <= 0) return;
+  const int nti = (rest + OZ_M - 1) / OZ_M, ntc = (rest + OZ_N - 1) / OZ_N;
+  constexpr int CW = LU_OUTER / OZ_N;
   static std::atomic<unsigned long long> attr{0};
   static int sms = 0;
   once_per_device(attr, [] {
@@ -576,9 +774,9 @@ inline void oz_apply(const OzSet& cur, const OzSet& prev, const OzStride& st, Ba
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   });
-  const long long tiles = (long long)nti * ntc * nsys;
+  const long long tiles = corner ? (long long)(CW * nti + std::max(0, ntc - CW)) * nsys : oz_tiles(rest, nsys);
   const int grid = (int)std::min<long long>(tiles, sms > 0 ? sms : 148);
-  oz_update_kernel<<<grid, OZ_THREADS, OZ_SMEM, stream>>>(b, k0, cur, prev, st, nsys, status, tl.ti0, nti, tj0, ntc);
+  oz_update_kernel<<<grid, OZ_THREADS, OZ_SMEM, stream>>>(b, k0, cur, prev, st, nsys, status, nti, ntc, corner ? 1 : 0);
   ++launches;
 }
 
