@@ -1735,11 +1735,10 @@ int nemoh_b200_free_surface(nemoh_ctx* c, double period, int npts, const double*
       CK(cudaMemsetAsync(base + o_p, 0, (size_t)npts * np * sizeof(double2), st));
       const dim3 grid((npts + FS_POINTS - 1) / FS_POINTS, (N + FS_PANELS - 1) / FS_PANELS);
       auto args = [&](auto kernel) {
-        kernel<<<grid, FS_POINTS, 0, st>>>(g, reinterpret_cast<const OmegaParams*>(base + o_om),
-                                           c->d_rec.as<PanelRec>(), N, reinterpret_cast<const double2*>(base + o_xy),
-                                           npts, np, reinterpret_cast<const double2*>(base + o_b),
-                                           reinterpret_cast<const double2*>(base + o_s),
-                                           reinterpret_cast<double2*>(base + o_p));
+        kernel<<<grid, FS_POINTS, fs_smem(np), st>>>(
+            g, reinterpret_cast<const OmegaParams*>(base + o_om), c->d_rec.as<PanelRec>(), N,
+            reinterpret_cast<const double2*>(base + o_xy), npts, np, reinterpret_cast<const double2*>(base + o_b),
+            reinterpret_cast<const double2*>(base + o_s), reinterpret_cast<double2*>(base + o_p));
       };
       if (fd) args(freesurface_kernel<true>);
       else args(freesurface_kernel<false>);
@@ -1779,11 +1778,11 @@ int nemoh_b200_irf(nemoh_ctx* c, int nw, const double* w, int nrad, int nint, co
     CK(cudaMemcpyAsync(dA, added_mass, nc * sizeof(double), cudaMemcpyHostToDevice, st));
     const unsigned chunks = (npair + IRF_CH - 1) / IRF_CH;
     if (ntime > 0) {
-      irf_kernel<<<dim3((ntime + IRF_THREADS - 1) / IRF_THREADS, chunks), IRF_THREADS, 0, st>>>(nw, dw, npair, dB,
-                                                                                                 ntime, dt, dK);
+      irf_kernel<<<(ntime + IRF_THREADS - 1) / IRF_THREADS * chunks, IRF_THREADS, 0, st>>>(nw, dw, npair, dB, ntime,
+                                                                                           dt, dK);
       LAUNCHED(c);
     }
-    irf_added_mass_kernel<<<dim3((nw + IRF_THREADS - 1) / IRF_THREADS, chunks), IRF_THREADS, 0, st>>>(
+    irf_added_mass_kernel<<<nw * chunks, IRF_THREADS, 0, st>>>(
         nw, dw, npair, dA, ntime, dt, dK, dcm);
     LAUNCHED(c);
     irf_average_kernel<<<(npair + 127) / 128, 128, 0, st>>>(nw, npair, dcm, dai);

@@ -151,13 +151,13 @@ constexpr int ASM_TJ = 32;
 #ifndef ASM_MINB_RANKINE
 #define ASM_MINB_RANKINE 3
 #endif
-// CTAs per SM of the wave pass (128 and 102 registers at most): measured on the barge
-// step, the finite-depth pass is fastest at 4 (at 5 its spills double and the
-// assembly takes 1.8 ms more); the deep-water pass spills the same at 96
-// registers as at 128 (its stack holds local arrays), and 5 CTAs save about
-// 0.5 ms of the step's assembly
+// CTAs per SM of the wave pass (102 registers at most): measured on the barge step,
+// the finite-depth pass takes 28.7 ms of assembly at 5, 30.0 at 4, 34.2 at 3 and
+// 30.1 at 6 (more warps hide the table gathers until the spills take the cache
+// from them); the deep-water pass spills the same at 96 registers as at 128 (its
+// stack holds local arrays), and 5 CTAs save about 0.5 ms of the step's assembly
 #ifndef ASM_MINB_WAVE_FD
-#define ASM_MINB_WAVE_FD 4
+#define ASM_MINB_WAVE_FD 5
 #endif
 #ifndef ASM_MINB_WAVE_INFD
 #define ASM_MINB_WAVE_INFD 5
@@ -441,6 +441,15 @@ __global__ void __launch_bounds__(WS_THREADS, FD ? ASM_MINB_WAVE_FD : ASM_MINB_W
     }
   };
   auto live = [&](int i, int j) { return i < na && j < nb && !(diag && i > j); };
+  if (rk) {
+    // the tile's and its transpose's Rankine parts come into L2 while the waves are
+    // evaluated: one thread per eight rows (128 bytes) of a column, half and class
+    const int cls = threadIdx.x >> 6, half = (threadIdx.x >> 5) & 1, col = (threadIdx.x & 31) >> 1;
+    const int seg = (threadIdx.x & 1) * 8;
+    const int r0 = half ? b0 : a0, c0 = half ? a0 : b0, nr = half ? nb : na, nc = half ? na : nb;
+    if (cls < NJJ && col < nc && seg < nr)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(rk + cls * NN + (r0 + seg) + (long long)N * (c0 + col)));
+  }
 #pragma unroll 1
   for (int q = threadIdx.x; q < WS_T * WS_T; q += WS_THREADS) {
     const int i = q % WS_T, j = q / WS_T;
@@ -452,11 +461,11 @@ __global__ void __launch_bounds__(WS_THREADS, FD ? ASM_MINB_WAVE_FD : ASM_MINB_W
     if (!lv) {
     } else if (PI.zg < g.zer && PJ.zg < g.zer) {
       if (FD) {
-        if (!wave_fd_sym(g, som, PI, PJ, NJJ, both, oij, oji)) {
-          set_status(g.status, ST_AKZ_UNDEFINED);
-          oij = oji = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
-        }
+        // the images first, while nothing of the tabulated part is live: their
+        // loop keeps to the registers
+        oij = oji = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
         fd_images_pair(g, som, PI, PJ, NJJ, both, oij, oji);
+        if (!wave_fd_sym_add(g, som, PI, PJ, NJJ, both, oij, oji)) set_status(g.status, ST_AKZ_UNDEFINED);
       } else {
         wave_infd_both(g, som, PI, PJ, NJJ, both, oij, oji);
       }

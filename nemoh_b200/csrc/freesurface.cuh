@@ -112,23 +112,30 @@ NB_HD __forceinline__ void field_green(const GreenCtx& g, const OmegaParams& om,
 }
 
 constexpr int FS_POINTS = 128;
-constexpr int FS_PANELS = 128;
+constexpr int FS_PANELS = 64;   // panels of a CTA: short, so that the grid's last wave is a small part
 constexpr int FS_MAXP = 16;
+// CTAs per SM (128 registers): a field point's sums wait in shared memory, so that
+// the Green functions have the registers; with the sums of 16 problems in registers
+// (255 and spills) two CTAs of four warps fitted an SM and the gathers' latency
+// bound the kernel. 10,201 points x 2,400 panels x 9 problems at 50 m depth, the
+// whole call: 10.0 to 7.9 ms (3 CTAs 8.1, 5 CTAs 8.1), and 7.2 ms with 64 panels
+// a CTA instead of 128 (32: 7.5, 200: 9.0).
+constexpr int FS_MINB = 4;
+inline int fs_smem(int nprob) { return nprob * FS_POINTS * (int)sizeof(double2); }
 
 // phi (npts x nprob complex, zeroed) += potential of the panels of chunk blockIdx.y
 template <bool FD>
-__global__ void __launch_bounds__(FS_POINTS)
+__global__ void __launch_bounds__(FS_POINTS, FS_MINB)
     freesurface_kernel(GreenCtx g, const OmegaParams* __restrict__ omp, const PanelRec* __restrict__ rec, int nfa,
                        const double2* __restrict__ xy, int npts, int nprob, const double2* __restrict__ zigb,
                        const double2* __restrict__ zigs, double2* phi) {
+  extern __shared__ double2 pot[];   // [nprob][FS_POINTS]: each thread its own column
   __shared__ PanelRec sp[ASM_TJ];
   __shared__ OmegaParams som;
   stage_params(omp, &som);
   const int q = blockIdx.x * FS_POINTS + threadIdx.x;
   const double XPO = q < npts ? xy[q].x : 0., YPO = q < npts ? xy[q].y : 0.;
-  double pot1[FS_MAXP], pot2[FS_MAXP];
-#pragma unroll
-  for (int p = 0; p < FS_MAXP; ++p) pot1[p] = pot2[p] = 0.;
+  for (int p = 0; p < nprob; ++p) pot[p * FS_POINTS + threadIdx.x] = make_double2(0., 0.);
   const int jbeg = blockIdx.y * FS_PANELS, jend = min(nfa, jbeg + FS_PANELS);
   for (int j0 = jbeg; j0 < jend; j0 += ASM_TJ) {
     const int nj = min(ASM_TJ, jend - j0);
@@ -141,29 +148,29 @@ __global__ void __launch_bounds__(FS_POINTS)
       double SP1, SP2, SM1, SM2;
       field_green<FD>(g, som, XPO, YPO, 0., sp[jj], SP1, SP2, SM1, SM2);
       const int J = j0 + jj;
-#pragma unroll
-      for (int p = 0; p < FS_MAXP; ++p) {
-        if (p >= nprob) break;
+      // with symmetry: the halves of the panel and of its mirror image
+      const double A1 = (SP1 + SM1) * 0.5, A2 = (SP2 + SM2) * 0.5, B1 = (SP1 - SM1) * 0.5, B2 = (SP2 - SM2) * 0.5;
+#pragma unroll 4
+      for (int p = 0; p < nprob; ++p) {
         const double2 b = zigb[(long long)p * nfa + J];
+        double2 v = pot[p * FS_POINTS + threadIdx.x];
         if (g.nsymy == 0) {
-          pot1[p] += b.x * SP1 - b.y * SP2;
-          pot2[p] += b.x * SP2 + b.y * SP1;
+          v.x += b.x * SP1 - b.y * SP2;
+          v.y += b.x * SP2 + b.y * SP1;
         } else {
           const double2 s = zigs[(long long)p * nfa + J];
-          const double C1 = b.x * (SP1 + SM1) + s.x * (SP1 - SM1), D1 = b.y * (SP2 + SM2) + s.y * (SP2 - SM2);
-          const double C2 = b.x * (SP2 + SM2) + s.x * (SP2 - SM2), D2 = b.y * (SP1 + SM1) + s.y * (SP1 - SM1);
-          pot1[p] += (C1 - D1) * 0.5;
-          pot2[p] += (C2 + D2) * 0.5;
+          v.x += (b.x * A1 + s.x * B1) - (b.y * A2 + s.y * B2);
+          v.y += (b.x * A2 + s.x * B2) + (b.y * A1 + s.y * B1);
         }
+        pot[p * FS_POINTS + threadIdx.x] = v;
       }
     }
   }
   if (q >= npts) return;
-#pragma unroll
-  for (int p = 0; p < FS_MAXP; ++p) {
-    if (p >= nprob) break;
-    atomicAdd(&phi[q + (long long)npts * p].x, pot1[p]);
-    atomicAdd(&phi[q + (long long)npts * p].y, pot2[p]);
+  for (int p = 0; p < nprob; ++p) {
+    const double2 v = pot[p * FS_POINTS + threadIdx.x];
+    atomicAdd(&phi[q + (long long)npts * p].x, v.x);
+    atomicAdd(&phi[q + (long long)npts * p].y, v.y);
   }
 }
 

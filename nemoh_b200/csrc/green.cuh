@@ -43,6 +43,22 @@ NB_HD __forceinline__ void set_status(int* st, int code) {
 #endif
 }
 
+// 1 / sqrt(x) for x in the normal range: the hardware's approximation (2^-20)
+// and one third-order step y (1 + h / 2 + 3 h^2 / 8), h = 1 - x y^2, whose
+// remainder is below 2^-58; about half the instructions of the library's rsqrt,
+// which also handles what a squared distance cannot be. Against it, the barge
+// step's assembly: 35.2 to 33.0 ms.
+NB_HD __forceinline__ double rsqrt3(double x) {
+#ifdef __CUDA_ARCH__
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = fma(-(x * y), y, 1.);
+  return fma(fma(0.375, h, 0.5), h * y, y);
+#else
+  return rsqrt(x);
+#endif
+}
+
 // --- GG(Z,CEX): ELEMENTARY_FNS.f90:31-81 ----------------------------------
 NB_HD __noinline__ cplx GG(cplx Z, cplx CEX) {
   const cplx IPI = mk(0., 3.14159265);
@@ -351,12 +367,22 @@ NB_HD __noinline__ void wave_infd_fs(const OmegaParams& om, double XGI, double Y
   w.FS1 *= s; w.FS2 *= s; w.VSX1 *= s; w.VSX2 *= s; w.VSY1 *= s; w.VSY2 *= s; w.VSZ1 *= s; w.VSZ2 *= s;
 }
 
+// 1 / DD with DD = sqrt(RRR^2 + ZZZ^2), 0 where the reference's DD > EPS fails:
+// decided exactly on the rounded square (the square root is monotone, T2 the
+// largest double whose root is <= EPS), so one reciprocal square root replaces
+// the exactly rounded root and the division by it
+NB_HD __forceinline__ double inverse_distance(double RRR2, double ZZZ, double T2) {
+  const double x = XADD(RRR2, XMUL(ZZZ, ZZZ));
+  const double ri = rsqrt3(x);
+  return x > T2 ? ri : 0.;
+}
+
 // --- VNSINFD tabulated branch, both reflections (:271-382) ----------------
 // AKZ depends on the depths only, so its stencil is shared by BX = +1 and -1.
 NB_HD __forceinline__ void wave_infd_pair(const GreenCtx& g, const OmegaParams& om, double XGI, double YGI,
                                                double ZMIII, const PanelRec& P, int NJJ, WaveJJ* w) {
   const double PI = 3.141592653589793, PI4 = 0.7853981633974483, DPI = 2. * PI, EPS = 0.0001;
-  const double AK0 = om.k0;
+  const double AK0 = om.k0, IAK0 = 1. / AK0;
   const double ZZZ = XADD(ZMIII, P.zg);
   const double AKZ = XMUL(AK0, ZZZ);
   if (AKZ > -1.5E-6) {
@@ -372,12 +398,8 @@ NB_HD __forceinline__ void wave_infd_pair(const GreenCtx& g, const OmegaParams& 
     const double dx = XSUB(XGI, P.xg), dy = XSUB(YGI, YMJJJ);
     const double RRR = XSQRT(XADD(XMUL(dx, dx), XMUL(dy, dy)));
     const double AKR = XMUL(AK0, RRR);
-    const double DD = XSQRT(XADD(XMUL(RRR, RRR), XMUL(ZZZ, ZZZ)));
-    double PSURR = 0.;
-    if (DD > EPS) {
-      const double it = 1. / (AK0 * DD);
-      PSURR = PI * it * it * it;
-    }
+    const double it = IAK0 * inverse_distance(XMUL(RRR, RRR), ZZZ, g.ro_eps2);
+    const double PSURR = PI * it * it * it;
     double PD1Z, PD2Z, VZ1, VZ2, PD1X = 0., PD2X = 0., VR1 = 0., VR2 = 0.;
     if (AKZ > -16.) {
       if (AKR < 99.7) {
@@ -525,49 +547,119 @@ struct FdImage {
   double PD1Z, PD2Z, VZ2, PD1X, VR2, PSR;
 };
 
-NB_HD __forceinline__ void fd_image(const GreenCtx& g, double AM0, double AKR, double RRR, double ZZZ, double AKZ,
-                                         const Stencil& sx, const Stencil& sz, bool tab, double PSK, double SCK,
-                                         double SCDS, double SSDS, FdImage& m) {
-  const double PI = 3.141592653589793, EPS = 0.0001;
-  const double DD = XSQRT(XADD(XMUL(RRR, RRR), XMUL(ZZZ, ZZZ)));
-  double PSURR = 0.;
-  m.PSR = 0.;
-  if (DD > EPS) {
-    const double it = 1. / (AM0 * DD);
-    m.PSR = PI * it;
-    PSURR = m.PSR * it * it;
+// coefficients of the asymptotic form beyond the tables (AKR >= 99.7), out of line
+// so that their temporaries cost the tabulated pairs nothing
+struct FarCoeffs {
+  double PSK, SCK, SCDS, SSDS;
+};
+NB_HD __noinline__ void far_coeffs(double AKR, FarCoeffs& c) {
+  const double PI = 3.141592653589793, PI4 = 0.7853981633974483, DPI = 2. * PI;
+  const double SQ = sqrt(DPI / AKR);
+  double SIK, CSK;
+  sincos(AKR - PI4, &SIK, &CSK);
+  c.PSK = PI * SQ * SIK;
+  c.SCK = SQ * CSK;
+  const double DSK = 0.5 / AKR;
+  c.SCDS = PI * SQ * (CSK - DSK * SIK);
+  c.SSDS = SQ * (SIK + DSK * CSK);
+}
+
+// IAM0 = 1 / AM0, RRR2 the rounded square of RRR; far: used when !tab
+NB_HD __forceinline__ void fd_image(const GreenCtx& g, double IAM0, double AKR, double RRR2, double ZZZ, double AKZ,
+                                         const Stencil& sx, const Stencil& sz, bool tab, const FarCoeffs& far,
+                                         FdImage& m) {
+  const double PI = 3.141592653589793;
+  const double it = IAM0 * inverse_distance(RRR2, ZZZ, g.ro_eps2);
+  m.PSR = PI * it;
+  if (AKZ > -16. && tab) {
+    const double4 t = interp4(g, sx, sz);
+    m.PD1X = t.x;
+    m.PD1Z = t.y;
+    m.PD2Z = t.w;
+    m.VZ2 = t.w;
+    m.VR2 = -t.z;
+    return;
   }
+  const double PSURR = m.PSR * it * it;
+  m.PD1Z = PSURR * AKZ;
+  m.PD1X = -PSURR * AKR;
+  m.PD2Z = 0.;
+  m.VR2 = 0.;
   if (AKZ > -16.) {
-    double PD1X, PD2X;
-    if (tab) {
-      const double4 t = interp4(g, sx, sz);
-      PD1X = t.x; m.PD1Z = t.y; PD2X = t.z; m.PD2Z = t.w;
-    } else {
-      const double EPZ = exp(AKZ);
-      m.PD1Z = PSURR * AKZ - PSK * EPZ;
-      m.PD2Z = EPZ * SCK;
-      PD1X = -PSURR * AKR - EPZ * SCDS;
-      PD2X = EPZ * SSDS;
+    const double EPZ = exp(AKZ);
+    m.PD1Z -= far.PSK * EPZ;
+    m.PD2Z = EPZ * far.SCK;
+    m.PD1X -= EPZ * far.SCDS;
+    m.VR2 = -(EPZ * far.SSDS);
+  }
+  m.VZ2 = m.PD2Z;
+}
+
+// --- VNSFD tabulated branch: the sums over the four images -------------------
+// Per reflection b (BX = +1, -1): the sums of PD1Z - PSR, PD2Z, PD1X and VR2,
+// and of PD1Z and VZ2 with the signs (+ - + -) of the z gradient of (I, J) and
+// (+ + - -) of (J, I). The image depths Z[k] (AKZ[k] = AM0 Z[k]) depend on the
+// panels' depths only, so both reflections share an image's depth stencil; |Z[0]|
+// is the smallest, so AKZ[0] <= -16 puts every image in the far branch. Image by
+// image, with both reflections' sums live, keeps fewer values live than
+// reflection by reflection with four stencils (barge step's assembly 33.0 to 28.3
+// ms, together with the images' loop in front of it and five CTAs per SM).
+struct FdSums {
+  double f1, f2, x1, x2, zp1, zq1, zp2, zq2;
+  double R2;       // RRR^2
+  bool away;       // RRR > EPS
+  NB_HD __forceinline__ double iR() const { return away ? rsqrt3(R2) : 0.; }
+};
+
+NB_HD __forceinline__ void fd_sums(const GreenCtx& g, double AM0, double XI, double YI, double XJ, double YJ,
+                                        const double* Z, const double* AKZ, int NJJ, FdSums* o) {
+  const double EPS = 0.0001, IAM0 = 1. / AM0;
+  const bool near = AKZ[0] > -16.;
+  double AKR[2];
+  Stencil sx[2];
+  bool tab[2];
+  FarCoeffs far[2];
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    o[b].f1 = o[b].f2 = o[b].x1 = o[b].x2 = o[b].zp1 = o[b].zq1 = o[b].zp2 = o[b].zq2 = 0.;
+    if (b >= NJJ) break;
+    const double dx = XSUB(XI, XJ), dy = XSUB(YI, b ? -YJ : YJ);
+    const double RRR = XSQRT(XADD(XMUL(dx, dx), XMUL(dy, dy)));
+    o[b].R2 = XMUL(RRR, RRR);
+    AKR[b] = XMUL(AM0, RRR);
+    tab[b] = AKR[b] < 99.7;
+    o[b].away = RRR > EPS;
+    sx[b] = Stencil{2, 0., 0., 0.};
+    if (near) {
+      if (tab[b]) stencil_x(g, AKR[b], sx[b]);
+      else far_coeffs(AKR[b], far[b]);
     }
-    m.VZ2 = m.PD2Z;
-    m.PD1X = PD1X;
-    m.VR2 = -PD2X;
-  } else {
-    m.PD1Z = PSURR * AKZ;
-    m.PD2Z = 0.;
-    m.VZ2 = 0.;
-    m.PD1X = -PSURR * AKR;
-    m.VR2 = 0.;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double sp = (k & 1) ? -1. : 1., sq = (k < 2) ? 1. : -1.;
+    Stencil sz{2, 0., 0., 0.};
+    if (AKZ[k] > -16. && (tab[0] || (NJJ == 2 && tab[1]))) stencil_z(g, AKZ[k], sz);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      if (b >= NJJ) break;
+      FdImage m;
+      fd_image(g, IAM0, AKR[b], o[b].R2, Z[k], AKZ[k], sx[b], sz, tab[b], far[b], m);
+      o[b].f1 += m.PD1Z - m.PSR;
+      o[b].f2 += m.PD2Z;
+      o[b].x1 += m.PD1X;
+      o[b].x2 += m.VR2;
+      o[b].zp1 += sp * m.PD1Z;
+      o[b].zq1 += sq * m.PD1Z;
+      o[b].zp2 += sp * m.VZ2;
+      o[b].zq2 += sq * m.VZ2;
+    }
   }
 }
 
-// --- VNSFD tabulated branch, both reflections ------------------------------
-// The four image depths Z1..Z4 (and their AKZ stencils) depend on the depths
-// only and are shared by BX = +1 and -1. |Z1| is the smallest of the four,
-// so AKZ1 <= -16 puts every image in the far branch.
+// one order of a pair, both reflections
 NB_HD __forceinline__ void wave_fd_pair(const GreenCtx& g, const OmegaParams& om, double XGI, double YGI,
                                              double ZMIII, const PanelRec& P, int NJJ, WaveJJ* w) {
-  const double PI = 3.141592653589793, PI4 = 0.7853981633974483, DPI = 2. * PI, EPS = 0.0001;
   const double AM0 = om.k0, H = om.h;
   const double COF1 = om.coe3 * P.aire, COF2 = om.coe4 * P.aire;
   const double COF3 = AM0 * COF1, COF4 = AM0 * COF2;
@@ -588,58 +680,23 @@ NB_HD __forceinline__ void wave_fd_pair(const GreenCtx& g, const OmegaParams& om
     w[0] = w[1] = WaveJJ{0, 0, 0, 0, 0, 0, 0, 0};
     return;
   }
-  const bool near = AKZ[0] > -16.;
-  Stencil sz[4];
-  bool have_sz = false;
-#pragma unroll 1
-  for (int b = 0; b < NJJ; ++b) {
-    const double YMJJJ = b ? -P.yg : P.yg;
-    const double dx = XSUB(XGI, P.xg), dy = XSUB(YGI, YMJJJ);
-    const double RRR = XSQRT(XADD(XMUL(dx, dx), XMUL(dy, dy)));
-    const double AKR = XMUL(AM0, RRR);
-    const bool tab = AKR < 99.7;
-    Stencil sx{2, 0., 0., 0.};
-    double PSK = 0., SCK = 0., SCDS = 0., SSDS = 0.;
-    if (near) {
-      if (tab) {
-        stencil_x(g, AKR, sx);
-        if (!have_sz) {
+  FdSums s[2];
+  fd_sums(g, AM0, XGI, YGI, P.xg, P.yg, Z, AKZ, NJJ, s);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (AKZ[k] > -16.) stencil_z(g, AKZ[k], sz[k]);
-          have_sz = true;
-        }
-      } else {
-        const double SQ = sqrt(DPI / AKR);
-        double SIK, CSK;
-        sincos(AKR - PI4, &SIK, &CSK);
-        PSK = PI * SQ * SIK;
-        SCK = SQ * CSK;
-        const double DSK = 0.5 / AKR;
-        SCDS = PI * SQ * (CSK - DSK * SIK);
-        SSDS = SQ * (SIK + DSK * CSK);
-      }
-    }
-    FdImage m[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) fd_image(g, AM0, AKR, RRR, Z[k], AKZ[k], sx, sz[k], tab, PSK, SCK, SCDS, SSDS, m[k]);
+  for (int b = 0; b < 2; ++b) {
+    if (b >= NJJ) break;
     WaveJJ& o = w[b];
-    o.FS1 = COF1 * ((m[0].PD1Z + m[1].PD1Z + m[2].PD1Z + m[3].PD1Z) - m[0].PSR - m[1].PSR - m[2].PSR - m[3].PSR);
-    o.FS2 = COF2 * (m[0].PD2Z + m[1].PD2Z + m[2].PD2Z + m[3].PD2Z);
-    if (RRR > EPS) {
-      const double C1V3 = -COF3 * (m[0].PD1X + m[1].PD1X + m[2].PD1X + m[3].PD1X);
-      const double C2V3 = COF4 * (m[0].VR2 + m[1].VR2 + m[2].VR2 + m[3].VR2);
-      const double iR = 1. / RRR;
-      const double CVX = dx * iR, CVY = dy * iR;
-      o.VSX1 = C1V3 * CVX;
-      o.VSX2 = C2V3 * CVX;
-      o.VSY1 = C1V3 * CVY;
-      o.VSY2 = C2V3 * CVY;
-    } else {
-      o.VSX1 = o.VSX2 = o.VSY1 = o.VSY2 = 0.;
-    }
-    o.VSZ1 = COF3 * (m[0].PD1Z - m[1].PD1Z + m[2].PD1Z - m[3].PD1Z);
-    o.VSZ2 = COF4 * (m[0].VZ2 - m[1].VZ2 + m[2].VZ2 - m[3].VZ2);
+    o.FS1 = COF1 * s[b].f1;
+    o.FS2 = COF2 * s[b].f2;
+    const double C1V3 = -COF3 * s[b].x1, C2V3 = COF4 * s[b].x2;
+    const double iR = s[b].iR();
+    const double CVX = XSUB(XGI, P.xg) * iR, CVY = XSUB(YGI, b ? -P.yg : P.yg) * iR;
+    o.VSX1 = C1V3 * CVX;
+    o.VSX2 = C2V3 * CVX;
+    o.VSY1 = C1V3 * CVY;
+    o.VSY2 = C2V3 * CVY;
+    o.VSZ1 = COF3 * s[b].zp1;
+    o.VSZ2 = COF4 * s[b].zp2;
   }
 }
 
@@ -674,9 +731,9 @@ NB_HD __forceinline__ void wave_sym_add(const OmegaParams& om, double aire, doub
   o.dm_im += sgn * D2;
 }
 
-NB_HD __forceinline__ bool wave_fd_sym(const GreenCtx& g, const OmegaParams& om, const PanelRec& PI,
-                                            const PanelRec& PJ, int NJJ, bool both, PairOut& oij, PairOut& oji) {
-  const double PI_ = 3.141592653589793, PI4 = 0.7853981633974483, DPI = 2. * PI_, EPS = 0.0001;
+// (wave_fd_sym_add adds to the outputs, in which the caller has the images.)
+NB_HD __forceinline__ bool wave_fd_sym_add(const GreenCtx& g, const OmegaParams& om, const PanelRec& PI,
+                                                const PanelRec& PJ, int NJJ, bool both, PairOut& oij, PairOut& oji) {
   const double AM0 = om.k0, H = om.h;
   const double H2 = XMUL(2., H), H4 = XMUL(4., H);
   double Z[4], AKZ[4];
@@ -691,70 +748,33 @@ NB_HD __forceinline__ bool wave_fd_sym(const GreenCtx& g, const OmegaParams& om,
     bad |= AKZ[k] > -1.5E-6;
   }
   if (bad) return false;
-  oij = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
-  oji = oij;
-  const bool near = AKZ[0] > -16.;
-  Stencil sz[4];
-  bool have_sz = false;
-#pragma unroll 1
-  for (int b = 0; b < NJJ; ++b) {
-    const double YMJJJ = b ? -PJ.yg : PJ.yg;
-    const double dx = XSUB(PI.xg, PJ.xg), dy = XSUB(PI.yg, YMJJJ);
-    const double RRR = XSQRT(XADD(XMUL(dx, dx), XMUL(dy, dy)));
-    const double AKR = XMUL(AM0, RRR);
-    const bool tab = AKR < 99.7;
-    Stencil sx{2, 0., 0., 0.};
-    double PSK = 0., SCK = 0., SCDS = 0., SSDS = 0.;
-    if (near) {
-      if (tab) {
-        stencil_x(g, AKR, sx);
-        if (!have_sz) {
+  FdSums s[2];
+  fd_sums(g, AM0, PI.xg, PI.yg, PJ.xg, PJ.yg, Z, AKZ, NJJ, s);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (AKZ[k] > -16.) stencil_z(g, AKZ[k], sz[k]);
-          have_sz = true;
-        }
-      } else {
-        const double SQ = sqrt(DPI / AKR);
-        double SIK, CSK;
-        sincos(AKR - PI4, &SIK, &CSK);
-        PSK = PI_ * SQ * SIK;
-        SCK = SQ * CSK;
-        const double DSK = 0.5 / AKR;
-        SCDS = PI_ * SQ * (CSK - DSK * SIK);
-        SSDS = SQ * (SIK + DSK * CSK);
-      }
-    }
-    // image by image into running sums: z gradients with the signs of
-    // (I, J) (+ - + -) and of (J, I) (+ + - -)
-    double s1z = 0., spsr = 0., s2z = 0., s1x = 0., s2r = 0., zp1 = 0., zq1 = 0., zp2 = 0., zq2 = 0.;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      FdImage m;
-      fd_image(g, AM0, AKR, RRR, Z[k], AKZ[k], sx, sz[k], tab, PSK, SCK, SCDS, SSDS, m);
-      const double sp = (k & 1) ? -1. : 1., sq = (k < 2) ? 1. : -1.;
-      s1z += m.PD1Z;
-      spsr += m.PSR;
-      s2z += m.PD2Z;
-      s1x += m.PD1X;
-      s2r += m.VR2;
-      zp1 += sp * m.PD1Z;
-      zq1 += sq * m.PD1Z;
-      zp2 += sp * m.VZ2;
-      zq2 += sq * m.VZ2;
-    }
-    const double F1 = s1z - spsr;
-    const double iR = RRR > EPS ? 1. / RRR : 0.;
-    const double sgn = b ? -1. : 1.;
-    wave_sym_add(om, PJ.aire, PI.xn, PI.yn, PI.zn, sgn, F1, s2z, s1x, s2r, zp1, zp2, dx * iR, dy * iR, oij);
+  for (int b = 0; b < 2; ++b) {
+    if (b >= NJJ) break;
+    const double sgn = b ? -1. : 1., iR = s[b].iR();
+    const double cx = XSUB(PI.xg, PJ.xg) * iR, cy = XSUB(PI.yg, b ? -PJ.yg : PJ.yg) * iR;
+    wave_sym_add(om, PJ.aire, PI.xn, PI.yn, PI.zn, sgn, s[b].f1, s[b].f2, s[b].x1, s[b].x2, s[b].zp1, s[b].zp2, cx, cy,
+                 oij);
     if (both)
-      wave_sym_add(om, PI.aire, PJ.xn, PJ.yn, PJ.zn, sgn, F1, s2z, s1x, s2r, zq1, zq2, -dx * iR,
-                   (b ? dy : -dy) * iR, oji);
+      wave_sym_add(om, PI.aire, PJ.xn, PJ.yn, PJ.zn, sgn, s[b].f1, s[b].f2, s[b].x1, s[b].x2, s[b].zq1, s[b].zq2, -cx,
+                   b ? cy : -cy, oji);
   }
   if (NJJ == 1) {   // one class: the minus entries equal the plus ones
     oij.sm_re = oij.sp_re; oij.sm_im = oij.sp_im; oij.dm_re = oij.dp_re; oij.dm_im = oij.dp_im;
     oji.sm_re = oji.sp_re; oji.sm_im = oji.sp_im; oji.dm_re = oji.dp_re; oji.dm_im = oji.dp_im;
   }
+  return true;
+}
+
+NB_HD __forceinline__ bool wave_fd_sym(const GreenCtx& g, const OmegaParams& om, const PanelRec& PI,
+                                            const PanelRec& PJ, int NJJ, bool both, PairOut& oij, PairOut& oji) {
+  const PairOut zero = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
+  PairOut a = zero, b = zero;
+  if (!wave_fd_sym_add(g, om, PI, PJ, NJJ, both, a, b)) return false;
+  oij = a;
+  oji = b;
   return true;
 }
 
@@ -797,6 +817,8 @@ NB_HD __forceinline__ void fd_image_sums(const GreenCtx& g, double H, const doub
     const double R = XSQRT(XADD(XMUL(o.dx[b], o.dx[b]), XMUL(o.dy[b], o.dy[b])));
     r2[b] = XMUL(R, R);
   }
+  // no image of a pair whose horizontal distance is above EPS can be closer
+  const bool far = r2[0] > T2 && (NJJ < 2 || r2[1] > T2);
 #pragma unroll 1
   for (int KE = 1; KE <= nexp1; ++KE) {
     const double A = ar[KE];
@@ -811,23 +833,22 @@ NB_HD __forceinline__ void fd_image_sums(const GreenCtx& g, double H, const doub
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       if (b >= NJJ) break;
-      double a[4], f = 0., sa = 0.;
+      double ri[4], a[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        // a select, not a branch: images closer than EPS contribute zero (the
-        // reciprocal of a zero distance is computed and dropped)
         const double RRk = XADD(r2[b], z2[k]);
-        const double ri0 = rsqrt(RRk);
-        const double ri = RRk > T2 ? ri0 : 0.;
-        f += ri;
-        a[k] = ri * ri * ri;
-        sa += a[k];
+        ri[k] = rsqrt3(RRk);
+        // images closer than EPS contribute zero (a select: the reciprocal of a
+        // zero distance is computed and dropped)
+        if (!far) ri[k] = RRk > T2 ? ri[k] : 0.;
+        a[k] = ri[k] * ri[k] * ri[k];
       }
-      const double p0 = zp[0] * a[0], p1 = zp[1] * a[1], p2 = zp[2] * a[2], p3 = zp[3] * a[3];
-      o.fs[b] += A * f;
-      o.sa[b] += A * sa;
-      o.m1[b] += A * ((p0 - p1) - (p2 - p3));
-      o.m2[b] += A * ((p0 + p1) + (p2 + p3));
+      // z a of the images whose sign the order exchanges (1, 2) and keeps (0, 3)
+      const double keep = zp[0] * a[0] + zp[3] * a[3], swap = zp[1] * a[1] + zp[2] * a[2];
+      o.fs[b] += A * ((ri[0] + ri[1]) + (ri[2] + ri[3]));
+      o.sa[b] += A * ((a[0] + a[1]) + (a[2] + a[3]));
+      o.m1[b] += A * (keep - swap);
+      o.m2[b] += A * (keep + swap);
     }
   }
 }
