@@ -220,20 +220,19 @@ inline void mixed_factor(MixedWork& w, double2* D, int n, int nsys, int* status,
         tc_prep(tg, bg, k0, ns, sg, launches);
         if (tc_prod) tc_products(tg, bg, k0, ns, sg, launches, status);
         if (!merge) {
-          tc_apply(tg, bg, k0, ns, sg, launches, status, TcTiles(), tc_persistent());
+          tc_apply(tg, bg, k0, ns, sg, launches, status, TcPart::all, tc_persistent());
           return;
         }
         auto it = deferred.find(s0);
         if (it != deferred.end() && it->second >= 0) {   // this panel's update and the deferred one
           const TcWork prev = slice(it->second);
-          tc_apply(tg, bg, k0, ns, sg, launches, status, TcTiles(), true, &prev);
+          tc_apply(tg, bg, k0, ns, sg, launches, status, TcPart::all, true, &prev);
           it->second = -1;
         } else if (kend + LU_OUTER < bg.n) {   // the next panel has columns beyond it: defer the bulk
-          tc_apply(tg, bg, k0, ns, sg, launches, status, TcTiles{0, -1, 0, 1}, true);
-          tc_apply(tg, bg, k0, ns, sg, launches, status, TcTiles{0, 1, 1, -1}, true);
+          tc_apply(tg, bg, k0, ns, sg, launches, status, TcPart::corner, true);
           deferred[s0] = set;
         } else {
-          tc_apply(tg, bg, k0, ns, sg, launches, status, TcTiles(), true);
+          tc_apply(tg, bg, k0, ns, sg, launches, status, TcPart::all, true);
         }
       },
       lanes, rg.host_ord, tc_prod);

@@ -348,14 +348,13 @@ __global__ void __launch_bounds__(128, 2) tc_update_kernel(BatchT<float2> b, int
                                                            const unsigned char* __restrict__ abuf,
                                                            const unsigned char* __restrict__ bbuf,
                                                            long long sys_bytes_a, long long sys_bytes_b, int* status,
-                                                           uint32_t idesc, int ti0, int tj0) {
+                                                           uint32_t idesc) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * TC_STAGE);   // full[2], empty[2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   __shared__ int s_ok;
   const int n = b.order(blockIdx.z), r1 = k0 + LU_OUTER, rest = n - r1;
-  // column tiles [tj0, tj0 + gridDim.x), row tiles [ti0, ti0 + gridDim.y)
-  const int tcol = blockIdx.x + tj0, trow = blockIdx.y + ti0;
+  const int tcol = blockIdx.x, trow = blockIdx.y;
   // a ragged batch's smaller systems leave the tiles beyond their order
   // (uniform per CTA, before any barrier or tensor-memory allocation)
   if (rest <= 0 || tcol * TC_T >= rest || trow * TC_T >= rest) return;
@@ -573,14 +572,19 @@ __device__ __forceinline__ void tc_store_b_rows(unsigned char* img, int row, con
 //   warps 2-5            read the accumulator (each warp the TMEM lane quarter
 //                        it may access, warp % 4), release it on acc_empty[buf]
 //                        and subtract it from A22.
-// Modes 1 and 2 are the panel's block products, written over their operand
-// (each tile is the only reader of its operand's tile) together with the
-// operand images of the trailing update, into iout:
-//   mode 1: L21 = A21 V, a row tile per tile (A: A21's images, B: V's);
-//   mode 2: conj(U12^T) = conj(A12^T) conj(W^T), a column tile of U12 per
-//           tile: accumulator row = column of U12, so each thread writes its
-//           column's B-image rows (A: the first half of A12's B images, B:
-//           conj(W^T)'s image).
+// With `wv` the launch forms the panel's block products, written over their
+// operand (each tile is the only reader of its operand's tile) together with the
+// operand images of the trailing update, over abuf and bbuf; a system's tiles are
+//   L21 = A21 V, nt row tiles (A: A21's images, B: V's), then
+//   conj(U12^T) = conj(A12^T) conj(W^T), nt column tiles of U12: accumulator
+//           row = column of U12, so each thread writes its column's B-image rows
+//           (A: the first half of A12's B images, B: conj(W^T)'s image). The
+//           matrix takes them through shared memory, a column's 32 entries a
+//           store: from the thread that holds the column each store touched 32
+//           lines (20 systems, 2,252 columns: 74 us, L21 31; both in one launch
+//           now 75).
+// `corner` takes the first row and column of tiles only, in one launch (53 us
+// there; a launch each took 64).
 // Every mbarrier wait is bounded; a role that times out raises the status,
 // flags the others through shared memory, and each role waits (bounded) for
 // the copies or MMAs it has in flight before the CTA frees its tensor memory.
@@ -588,12 +592,12 @@ __device__ __forceinline__ void tc_store_b_rows(unsigned char* img, int row, con
 constexpr int TCP_STAGES = 4;
 constexpr int TCP_THREADS = 192;
 constexpr int TCP_SMEM = TCP_STAGES * TC_STAGE + 256;
+constexpr int TCP_SMEM_PROD = TCP_SMEM + 4 * 32 * 33 * (int)sizeof(float2);   // with the columns' staging
 
 __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
-    BatchT<float2> b, int k0, const unsigned char* __restrict__ abuf, const unsigned char* __restrict__ bbuf,
-    long long sys_bytes_a, long long sys_bytes_b, int nt, int nsys, int* status, uint32_t idesc, int ti0, int nti,
-    int tj0, int ntc, const unsigned char* __restrict__ pabuf, const unsigned char* __restrict__ pbbuf, int mode,
-    unsigned char* iout, int f16) {
+    BatchT<float2> b, int k0, unsigned char* abuf, unsigned char* bbuf, long long sys_bytes_a, long long sys_bytes_b,
+    int nt, int nsys, int* status, uint32_t idesc, int corner, const unsigned char* __restrict__ pabuf,
+    const unsigned char* __restrict__ pbbuf, const unsigned char* __restrict__ wv, int f16) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TCP_STAGES * TC_STAGE);
   // bars: full[S], empty[S], acc_full[2], acc_empty[2]; then the TMEM address
@@ -603,16 +607,23 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[TCP_STAGES]);
   const uint32_t accf0 = smem_u32(&bars[2 * TCP_STAGES]), acce0 = smem_u32(&bars[2 * TCP_STAGES + 2]);
   const int r1 = k0 + LU_OUTER;
-  const long long total = (long long)nti * ntc * nsys;
+  const int per = wv ? 2 * nt : corner ? 2 * nt - 1 : nt * nt;   // tiles of a system
+  const long long total = (long long)per * nsys;
   // chunks per tile: the previous panel's images first (a merged update), then this panel's
   const int nch = pabuf ? 2 * TC_NCH : TC_NCH;
-  // tile t: system z, row tile trow in [ti0, ti0 + nti), column tile tcol in
-  // [tj0, tj0 + ntc); false beyond a ragged system's order
-  auto tile = [&](long long t, int& z, int& trow, int& tcol) {
-    z = (int)(t / ((long long)nti * ntc));
-    const int rem = (int)(t % ((long long)nti * ntc));
-    trow = ti0 + rem / ntc;
-    tcol = tj0 + rem % ntc;
+  // tile t: system z, row tile trow, column tile tcol; mode 0: update, 1: L21, 2: U12;
+  // false beyond a ragged system's order
+  auto tile = [&](long long t, int& z, int& trow, int& tcol, int& mode) {
+    z = (int)(t / per);
+    const int rem = (int)(t % per);
+    mode = wv ? (rem < nt ? 1 : 2) : 0;
+    if (wv || corner) {
+      trow = rem < nt ? rem : 0;
+      tcol = rem < nt ? 0 : rem - nt + (wv ? 0 : 1);
+    } else {
+      trow = rem / nt;
+      tcol = rem % nt;
+    }
     const int rest = b.order(z) - r1;
     return rest > 0 && trow * TC_T < rest && tcol * TC_T < rest;
   };
@@ -648,8 +659,8 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
     long long g = 0;   // chunks issued
     bool ok = true;
     for (long long t = blockIdx.x; t < total && ok && !s_err; t += gridDim.x) {
-      int z, trow, tcol;
-      if (!tile(t, z, trow, tcol)) continue;
+      int z, trow, tcol, mode;
+      if (!tile(t, z, trow, tcol, mode)) continue;
       for (int c = 0; c < nch; ++c) {
         // the previous panel's tiles are one tile further: its trailing block starts 128 earlier
         const bool prev = pabuf && c < TC_NCH;
@@ -661,13 +672,11 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
         const int q = (int)(g % TCP_STAGES);
         const long long r = g / TCP_STAGES;
         if (r > 0 && !(ok = mbar_wait(empty0 + 8 * q, (uint32_t)((r - 1) & 1)))) break;
-        if (mode == 2) {   // A: rows of A12's B image (column tile tcol), B: conj(W^T) (one tile)
-          const unsigned char* gt = abuf + z * sys_bytes_a + ((long long)tcol * TC_NCH + cc) * 2 * TC_BIMG;
-          tc_load_chunk_split(s0 + q * TC_STAGE, gt, gt + TC_BIMG, bbuf + z * sys_bytes_b + (long long)cc * 2 * TC_BIMG,
-                              full0 + 8 * q);
-        } else {
-          tc_load_chunk(s0 + q * TC_STAGE, ga, gb, full0 + 8 * q);
-        }
+        const unsigned char* gw = wv + z * (long long)TC_WV_BYTES + (long long)cc * 2 * TC_BIMG;
+        if (mode == 2)   // A: rows of A12's B image (column tile tcol), B: conj(W^T)
+          tc_load_chunk_split(s0 + q * TC_STAGE, gb, gb + TC_BIMG, gw, full0 + 8 * q);
+        else   // L21: B is V's image
+          tc_load_chunk(s0 + q * TC_STAGE, ga, mode == 1 ? gw + TC_W_BYTES : gb, full0 + 8 * q);
         ++g;
       }
     }
@@ -681,8 +690,8 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
     long long g = 0, i = 0;   // chunks consumed, tiles done
     bool ok = true;
     for (long long t = blockIdx.x; t < total && ok && !s_err; t += gridDim.x) {
-      int z, trow, tcol;
-      if (!tile(t, z, trow, tcol)) continue;
+      int z, trow, tcol, mode;
+      if (!tile(t, z, trow, tcol, mode)) continue;
       const int buf = (int)(i & 1);
       const long long u = i >> 1;
       if (u > 0 && !(ok = mbar_wait(acce0 + 8 * buf, (uint32_t)((u - 1) & 1)))) break;
@@ -725,8 +734,8 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
     bool ok = true;
     for (long long t = blockIdx.x; t < total; t += gridDim.x) {
       if (__shfl_sync(0xffffffffu, s_err, 0)) break;
-      int z, trow, tcol;
-      if (!tile(t, z, trow, tcol)) continue;
+      int z, trow, tcol, mode;
+      if (!tile(t, z, trow, tcol, mode)) continue;
       const int buf = (int)(i & 1);
       const bool got = mbar_wait(accf0 + 8 * buf, (uint32_t)((i >> 1) & 1));
       if (!(ok = __all_sync(0xffffffffu, got))) break;
@@ -767,12 +776,17 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * buf) : "memory");
         }
         if (mode == 2) {   // accumulator: Re U12(k0 + k, gr) at column k, -Im U12 at 128 + k
-          if (gr < n) {
-            float2* p = A + (k0 + 32 * q) + (long long)n * gr;
+          float2* tr = reinterpret_cast<float2*>(smem + TCP_SMEM) + lq * (32 * 33);   // [column][33]
 #pragma unroll
-            for (int j = 0; j < 32; ++j) p[j] = make_float2(__uint_as_float(vr[j]), -__uint_as_float(vi[j]));
-          }
-          tc_store_b_rows(iout + z * sys_bytes_a + ((long long)tcol * TC_NCH + 2 * q) * 2 * TC_BIMG, row, vr, vi, f16);
+          for (int j = 0; j < 32; ++j) tr[lane * 33 + j] = make_float2(__uint_as_float(vr[j]), -__uint_as_float(vi[j]));
+          __syncwarp();
+          const int g0 = gr - lane;   // the warp's first column
+          float2* p = A + (k0 + 32 * q + lane) + (long long)n * g0;
+#pragma unroll 8
+          for (int j = 0; j < 32; ++j)
+            if (g0 + j < n) p[(long long)n * j] = tr[j * 33 + lane];
+          __syncwarp();
+          tc_store_b_rows(bbuf + z * sys_bytes_b + ((long long)tcol * TC_NCH + 2 * q) * 2 * TC_BIMG, row, vr, vi, f16);
         } else if (gr < n && 32 * q < ncol) {
           float2* p = A + gr + (long long)n * (cbase + 32 * q);
           if (mode == 0) {
@@ -795,7 +809,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) tc_update_persistent_kernel(
           }
         }
         if (mode == 1)   // rows beyond the order are zero, as tc_prep_kernel writes them
-          tc_store_a_row(iout + z * sys_bytes_a + ((long long)trow * TC_NCH + 2 * q) * 2 * TC_AIMG, row, vr, vi, f16);
+          tc_store_a_row(abuf + z * sys_bytes_a + ((long long)trow * TC_NCH + 2 * q) * 2 * TC_AIMG, row, vr, vi, f16);
       }
       ++i;
     }
@@ -865,60 +879,55 @@ inline void tc_prep(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStream_t 
   ++launches;
 }
 
-// A rectangle of tiles of the trailing matrix: row tiles [ti0, ti0 + nti),
-// column tiles [tj0, tj0 + ntc) (a count < 0: to the last tile)
-struct TcTiles {
-  int ti0 = 0, nti = -1, tj0 = 0, ntc = -1;
-};
+enum class TcPart { all, corner };   // every tile of the trailing matrix, or its first row and column of tiles
 
-// The update of a rectangle of tiles of the trailing matrix from the images
-// tc_prep wrote; persistent: one CTA per SM walking the tiles (the default
-// form), else one tile per CTA. prev (persistent form only): the images of
+inline int tc_grid(long long tiles) {   // sets the kernel's attributes once per device
+  static std::atomic<unsigned long long> attr{0};
+  static int sms = 0;
+  once_per_device(attr, [] {
+    cudaFuncSetAttribute(tc_update_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TCP_SMEM_PROD);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  });
+  return (int)std::min<long long>(tiles, tc_grid_cap(sms > 0 ? sms : 148));
+}
+
+// The update of the trailing matrix, or of its corner, from the images tc_prep
+// wrote; persistent: one CTA per SM walking the tiles (the default form), else
+// one tile per CTA (all tiles). prev (persistent form only): the images of
 // the previous panel, whose update of these tiles was deferred and is merged
 // here (K = 256 in one accumulation: one read-modify-write of the tiles for
 // two panels).
 inline void tc_apply(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStream_t st, long long& launches,
-                     int* status, TcTiles tl, bool persistent, const TcWork* prev = nullptr) {
+                     int* status, TcPart part, bool persistent, const TcWork* prev = nullptr) {
   const int n = b.n, rest = n - k0 - LU_OUTER;
   if (rest <= 0) return;
   const int t = (n + TC_T - 1) / TC_T;
   const long long sa = (long long)t * TC_NCH * 2 * TC_AIMG, sb = (long long)t * TC_NCH * 2 * TC_BIMG;
   const int nt = (rest + TC_T - 1) / TC_T;
-  const int nti = std::min(tl.nti < 0 ? nt - tl.ti0 : tl.nti, nt - tl.ti0);
-  const int ntc = std::min(tl.ntc < 0 ? nt - tl.tj0 : tl.ntc, nt - tl.tj0);
-  if (nti <= 0 || ntc <= 0) return;
   const uint32_t idesc = tc_idesc(tc_split_f16());
-  if (persistent || prev) {
-    static std::atomic<unsigned long long> attr2{0};
-    static int sms = 0;
-    once_per_device(attr2, [] {
-      cudaFuncSetAttribute(tc_update_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TCP_SMEM);
-      int dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    });
-    const long long tiles = (long long)nti * ntc * nsys;
-    const int grid = (int)std::min<long long>(tiles, tc_grid_cap(sms > 0 ? sms : 148));
+  if (persistent) {
+    const int corner = part == TcPart::corner;
+    const int grid = tc_grid((corner ? 2LL * nt - 1 : (long long)nt * nt) * nsys);
     tc_update_persistent_kernel<<<grid, TCP_THREADS, TCP_SMEM, st>>>(
-        b, k0, w.a, w.b, sa, sb, nt, nsys, status, idesc, tl.ti0, nti, tl.tj0, ntc, prev ? prev->a : nullptr,
-        prev ? prev->b : nullptr, 0, nullptr, 0);
+        b, k0, w.a, w.b, sa, sb, nt, nsys, status, idesc, corner, prev ? prev->a : nullptr,
+        prev ? prev->b : nullptr, nullptr, 0);
   } else {
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] {
       cudaFuncSetAttribute(tc_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
     });
-    tc_update_kernel<<<dim3(ntc, nti, nsys), 128, TC_SMEM, st>>>(b, k0, w.a, w.b, sa, sb, status, idesc, tl.ti0,
-                                                                 tl.tj0);
+    tc_update_kernel<<<dim3(nt, nt, nsys), 128, TC_SMEM, st>>>(b, k0, w.a, w.b, sa, sb, status, idesc);
   }
   ++launches;
 }
 
 // The panel's block products on the tensor cores (persistent form), from
-// the images tc_prep wrote of A21 and A12 before them: L21 = A21 V (every row
-// tile, one column tile) and U12 = W A12 (one row tile, every column tile),
-// each written over its operand; W and V from the panel's inverses
-// (panel_inv_kernel). Both write the trailing update's operand images of the
-// products over the operands' images (the update needs no tc_prep after).
+// the images tc_prep wrote of A21 and A12 before them: L21 = A21 V and
+// U12 = W A12, each written over its operand; W and V from the panel's inverses
+// (panel_inv_kernel). The trailing update's operand images of the products
+// replace the operands' images (the update needs no tc_prep after).
 inline void tc_products(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStream_t st, long long& launches,
                         int* status) {
   const int n = b.n, rest = n - k0 - LU_OUTER;
@@ -929,26 +938,9 @@ inline void tc_products(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStrea
   constexpr int PER = TC_T * TC_NCH / 128;
   if (tc_split_f16()) tc_prep_wv_kernel<true><<<dim3(2 * PER, 1, nsys), 128, 0, st>>>(b, k0, w.wv);
   else tc_prep_wv_kernel<false><<<dim3(2 * PER, 1, nsys), 128, 0, st>>>(b, k0, w.wv);
-  ++launches;
-  const uint32_t idesc = tc_idesc(tc_split_f16());
-  static std::atomic<unsigned long long> attr{0};
-  static int sms = 0;
-  once_per_device(attr, [] {
-    cudaFuncSetAttribute(tc_update_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TCP_SMEM);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  });
-  const int cap = tc_grid_cap(sms > 0 ? sms : 148);
-  const int f16 = tc_split_f16() ? 1 : 0;
-  // L21 = A21 V: A images of A21 (row tiles), the B image of V (tile 0)
-  tc_update_persistent_kernel<<<(int)std::min<long long>((long long)nt * nsys, cap), TCP_THREADS, TCP_SMEM, st>>>(
-      b, k0, w.a, w.wv + TC_W_BYTES, sa, TC_WV_BYTES, nt, nsys, status, idesc, 0, nt, 0, 1, nullptr, nullptr, 1, w.a,
-      f16);
-  // conj(U12^T) = conj(A12^T) conj(W^T): A from the B images of A12 (column
-  // tiles), B the image of conj(W^T) (tile 0)
-  tc_update_persistent_kernel<<<(int)std::min<long long>((long long)nt * nsys, cap), TCP_THREADS, TCP_SMEM, st>>>(
-      b, k0, w.b, w.wv, sb, TC_WV_BYTES, nt, nsys, status, idesc, 0, 1, 0, nt, nullptr, nullptr, 2, w.b, f16);
+  tc_update_persistent_kernel<<<tc_grid(2LL * nt * nsys), TCP_THREADS, TCP_SMEM_PROD, st>>>(
+      b, k0, w.a, w.b, sa, sb, nt, nsys, status, tc_idesc(tc_split_f16()), 0, nullptr, nullptr, w.wv,
+      tc_split_f16() ? 1 : 0);
   launches += 2;
 }
 
