@@ -217,7 +217,7 @@ inline void mixed_factor(MixedWork& w, double2* D, int n, int nsys, int* status,
         // operand images of the panel's columns and rows: with tc_prod those of
         // A21 and A12, from which the block products form L21 = A21 V and
         // U12 = W A12 together with their images; else those of L21 and U12
-        tc_prep(tg, bg, k0, ns, sg, launches);
+        tc_prep(tg, bg, k0, ns, sg, launches, tc_prod);
         if (tc_prod) tc_products(tg, bg, k0, ns, sg, launches, status);
         if (!merge) {
           tc_apply(tg, bg, k0, ns, sg, launches, status, TcPart::all, tc_persistent());

@@ -128,68 +128,7 @@ __device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& lo) {
   lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// Operand images of the outer update after the panel [k0, k0 + 128):
-// L21 = A[r1:n, k0:k0+128] and U12 = A[k0:k0+128, r1:n] with r1 = k0 + 128.
-// Thread per (row or column of the tile, chunk); blocks [0, na) do A, the rest B.
-template <bool F16>
-__global__ void __launch_bounds__(128) tc_prep_kernel(BatchT<float2> b, int k0, unsigned char* __restrict__ abuf,
-                                                       unsigned char* __restrict__ bbuf, long long sys_bytes_a,
-                                                       long long sys_bytes_b, int na) {
-  const int n = b.order(blockIdx.z), r1 = k0 + LU_OUTER, rest = n - r1;
-  if (rest <= 0) return;
-  const int nt = (rest + TC_T - 1) / TC_T;
-  const float2* A = b.sys(blockIdx.z);
-  const bool isA = (int)blockIdx.x < na;
-  const int q = (isA ? blockIdx.x : blockIdx.x - na) * blockDim.x + threadIdx.x;
-  if (q >= nt * TC_T * TC_NCH) return;
-  const int ch = q / (nt * TC_T), rr = q % (nt * TC_T);   // consecutive threads: consecutive rows/columns
-  const int t = rr / TC_T, row = rr % TC_T;
-  const int kb = k0 + ch * TC_KC;
-  float re[TC_KC], im[TC_KC];
-  if (isA) {
-    const int r = r1 + rr;
-#pragma unroll
-    for (int j = 0; j < TC_KC; ++j) {
-      const float2 v = (r < n) ? A[r + (long long)n * (kb + j)] : make_float2(0.f, 0.f);
-      re[j] = v.x;
-      im[j] = v.y;
-    }
-    unsigned char* img = abuf + blockIdx.z * sys_bytes_a + ((long long)t * TC_NCH + ch) * 2 * TC_AIMG;
-    uint4 h, l;
-    // k-groups: 0,1 = Re(k 0..15), 2,3 = Im(k 0..15)
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      split8<F16>((g < 2 ? re : im) + 8 * (g & 1), h, l);
-      *reinterpret_cast<uint4*>(img + tc_row_off(row, g)) = h;
-      *reinterpret_cast<uint4*>(img + TC_AIMG + tc_row_off(row, g)) = l;
-    }
-  } else {
-    const int c = r1 + rr;
-    const float2* col = A + (long long)n * c + kb;
-#pragma unroll
-    for (int j = 0; j < TC_KC; ++j) {
-      const float2 v = (c < n) ? col[j] : make_float2(0.f, 0.f);
-      re[j] = v.x;
-      im[j] = v.y;
-    }
-    float nim[TC_KC];
-#pragma unroll
-    for (int j = 0; j < TC_KC; ++j) nim[j] = -im[j];
-    unsigned char* img = bbuf + blockIdx.z * sys_bytes_b + ((long long)t * TC_NCH + ch) * 2 * TC_BIMG;
-    uint4 h, l;
-    // B row `row` (real parts of the result): [Br; -Bi]; row 128+row (imaginary parts): [Bi; Br]
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      split8<F16>((g < 2 ? re : nim) + 8 * (g & 1), h, l);
-      *reinterpret_cast<uint4*>(img + tc_row_off(row, g)) = h;
-      *reinterpret_cast<uint4*>(img + TC_BIMG + tc_row_off(row, g)) = l;
-      split8<F16>((g < 2 ? im : re) + 8 * (g & 1), h, l);
-      *reinterpret_cast<uint4*>(img + tc_row_off(TC_T + row, g)) = h;
-      *reinterpret_cast<uint4*>(img + TC_BIMG + tc_row_off(TC_T + row, g)) = l;
-    }
-  }
-}
-
+constexpr int TC_WV_CTAS = 2 * TC_T * TC_NCH / 128;
 // Images of the panel's W = inv(L11) and V = inv(U11), K = 128, in the
 // layout of tc_prep_kernel's, for the block products on the tensor cores:
 // V as the B tile of L21 = A21 V, and conj(W^T) as the B tile of
@@ -197,13 +136,11 @@ __global__ void __launch_bounds__(128) tc_prep_kernel(BatchT<float2> b, int k0, 
 // (its A operand, conj(A12^T), is the first half of A12's B image, and each
 // accumulator row is then one column of U12). Blocks [0, 8): W, [8, 16): V.
 template <bool F16>
-__global__ void __launch_bounds__(128) tc_prep_wv_kernel(BatchT<float2> b, int k0, unsigned char* __restrict__ wv) {
-  const int n = b.order(blockIdx.z);
-  if (k0 + LU_OUTER >= n) return;
+__device__ __forceinline__ void tc_prep_wv(const BatchT<float2>& b, unsigned char* __restrict__ wv, int blk) {
   const float2* P = b.pinv + (long long)blockIdx.z * PINV_SCRATCH;
-  constexpr int PER = TC_T * TC_NCH / 128;
-  const bool isW = (int)blockIdx.x < PER;
-  const int q = (isW ? blockIdx.x : blockIdx.x - PER) * 128 + threadIdx.x;   // < TC_T * TC_NCH
+  constexpr int PER = TC_WV_CTAS / 2;
+  const bool isW = blk < PER;
+  const int q = (isW ? blk : blk - PER) * 128 + threadIdx.x;   // < TC_T * TC_NCH
   const int ch = q / TC_T, row = q % TC_T, kb = ch * TC_KC;
   unsigned char* base = wv + blockIdx.z * TC_WV_BYTES;
   // only the 32 x 32 blocks of the triangle are formed (W's column block, and
@@ -245,6 +182,75 @@ __global__ void __launch_bounds__(128) tc_prep_wv_kernel(BatchT<float2> b, int k
 #pragma unroll
     for (int j = 0; j < TC_KC; ++j) nim[j] = -im[j];
     unsigned char* img = base + TC_W_BYTES + (long long)ch * 2 * TC_BIMG;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      split8<F16>((g < 2 ? re : nim) + 8 * (g & 1), h, l);
+      *reinterpret_cast<uint4*>(img + tc_row_off(row, g)) = h;
+      *reinterpret_cast<uint4*>(img + TC_BIMG + tc_row_off(row, g)) = l;
+      split8<F16>((g < 2 ? im : re) + 8 * (g & 1), h, l);
+      *reinterpret_cast<uint4*>(img + tc_row_off(TC_T + row, g)) = h;
+      *reinterpret_cast<uint4*>(img + TC_BIMG + tc_row_off(TC_T + row, g)) = l;
+    }
+  }
+}
+
+// Operand images of the outer update after the panel [k0, k0 + 128):
+// L21 = A[r1:n, k0:k0+128] and U12 = A[k0:k0+128, r1:n] with r1 = k0 + 128.
+// Thread per (row or column of the tile, chunk); blocks [0, na) do A, [na, 2 na) B
+// and, with wv, TC_WV_CTAS more those of W and V (as a launch of their own
+// 6.5 us a panel: 48 requests of 12 hulls, LU 3.23 to 3.10 ms).
+template <bool F16>
+__global__ void __launch_bounds__(128) tc_prep_kernel(BatchT<float2> b, int k0, unsigned char* __restrict__ abuf,
+                                                       unsigned char* __restrict__ bbuf, long long sys_bytes_a,
+                                                       long long sys_bytes_b, int na,
+                                                       unsigned char* __restrict__ wv) {
+  const int n = b.order(blockIdx.z), r1 = k0 + LU_OUTER, rest = n - r1;
+  if (rest <= 0) return;
+  if ((int)blockIdx.x >= 2 * na) {
+    tc_prep_wv<F16>(b, wv, blockIdx.x - 2 * na);
+    return;
+  }
+  const int nt = (rest + TC_T - 1) / TC_T;
+  const float2* A = b.sys(blockIdx.z);
+  const bool isA = (int)blockIdx.x < na;
+  const int q = (isA ? blockIdx.x : blockIdx.x - na) * blockDim.x + threadIdx.x;
+  if (q >= nt * TC_T * TC_NCH) return;
+  const int ch = q / (nt * TC_T), rr = q % (nt * TC_T);   // consecutive threads: consecutive rows/columns
+  const int t = rr / TC_T, row = rr % TC_T;
+  const int kb = k0 + ch * TC_KC;
+  float re[TC_KC], im[TC_KC];
+  if (isA) {
+    const int r = r1 + rr;
+#pragma unroll
+    for (int j = 0; j < TC_KC; ++j) {
+      const float2 v = (r < n) ? A[r + (long long)n * (kb + j)] : make_float2(0.f, 0.f);
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    unsigned char* img = abuf + blockIdx.z * sys_bytes_a + ((long long)t * TC_NCH + ch) * 2 * TC_AIMG;
+    uint4 h, l;
+    // k-groups: 0,1 = Re(k 0..15), 2,3 = Im(k 0..15)
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      split8<F16>((g < 2 ? re : im) + 8 * (g & 1), h, l);
+      *reinterpret_cast<uint4*>(img + tc_row_off(row, g)) = h;
+      *reinterpret_cast<uint4*>(img + TC_AIMG + tc_row_off(row, g)) = l;
+    }
+  } else {
+    const int c = r1 + rr;
+    const float2* col = A + (long long)n * c + kb;
+#pragma unroll
+    for (int j = 0; j < TC_KC; ++j) {
+      const float2 v = (c < n) ? col[j] : make_float2(0.f, 0.f);
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    float nim[TC_KC];
+#pragma unroll
+    for (int j = 0; j < TC_KC; ++j) nim[j] = -im[j];
+    unsigned char* img = bbuf + blockIdx.z * sys_bytes_b + ((long long)t * TC_NCH + ch) * 2 * TC_BIMG;
+    uint4 h, l;
+    // B row `row` (real parts of the result): [Br; -Bi]; row 128+row (imaginary parts): [Bi; Br]
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       split8<F16>((g < 2 ? re : nim) + 8 * (g & 1), h, l);
@@ -866,16 +872,19 @@ inline bool tc_enabled() {
   return on;
 }
 
-// operand images of the outer update after the panel [k0, k0+128)
-inline void tc_prep(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStream_t st, long long& launches) {
+// operand images of the outer update after the panel [k0, k0+128); products: of
+// the block products that come first, W's and V's too
+inline void tc_prep(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStream_t st, long long& launches,
+                    bool products) {
   const int n = b.n, rest = n - k0 - LU_OUTER;
   if (rest <= 0) return;
   const int t = (n + TC_T - 1) / TC_T;
   const long long sa = (long long)t * TC_NCH * 2 * TC_AIMG, sb = (long long)t * TC_NCH * 2 * TC_BIMG;
   const int nt = (rest + TC_T - 1) / TC_T;
   const int per = (nt * TC_T * TC_NCH + 127) / 128;
-  if (tc_split_f16()) tc_prep_kernel<true><<<dim3(2 * per, 1, nsys), 128, 0, st>>>(b, k0, w.a, w.b, sa, sb, per);
-  else tc_prep_kernel<false><<<dim3(2 * per, 1, nsys), 128, 0, st>>>(b, k0, w.a, w.b, sa, sb, per);
+  const dim3 grid(2 * per + (products ? TC_WV_CTAS : 0), 1, nsys);
+  if (tc_split_f16()) tc_prep_kernel<true><<<grid, 128, 0, st>>>(b, k0, w.a, w.b, sa, sb, per, w.wv);
+  else tc_prep_kernel<false><<<grid, 128, 0, st>>>(b, k0, w.a, w.b, sa, sb, per, w.wv);
   ++launches;
 }
 
@@ -935,13 +944,10 @@ inline void tc_products(TcWork& w, BatchT<float2> b, int k0, int nsys, cudaStrea
   const int t = (n + TC_T - 1) / TC_T;
   const long long sa = (long long)t * TC_NCH * 2 * TC_AIMG, sb = (long long)t * TC_NCH * 2 * TC_BIMG;
   const int nt = (rest + TC_T - 1) / TC_T;
-  constexpr int PER = TC_T * TC_NCH / 128;
-  if (tc_split_f16()) tc_prep_wv_kernel<true><<<dim3(2 * PER, 1, nsys), 128, 0, st>>>(b, k0, w.wv);
-  else tc_prep_wv_kernel<false><<<dim3(2 * PER, 1, nsys), 128, 0, st>>>(b, k0, w.wv);
   tc_update_persistent_kernel<<<tc_grid(2LL * nt * nsys), TCP_THREADS, TCP_SMEM_PROD, st>>>(
       b, k0, w.a, w.b, sa, sb, nt, nsys, status, tc_idesc(tc_split_f16()), 0, nullptr, nullptr, w.wv,
       tc_split_f16() ? 1 : 0);
-  launches += 2;
+  ++launches;
 }
 
 }  // namespace nb200
