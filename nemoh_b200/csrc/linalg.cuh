@@ -10,8 +10,10 @@
 //   lu_diag_kernel    factor A11 once per system, invert L11 and U11
 //   lu_panel_kernel   L21 <- A21 U11^-1, U12 <- L11^-1 A12, store factored A11
 //   zgemm_update      A22 <- A22 - L21 U12 over any rectangle of A22
-// The FP64 path updates the whole trailing matrix after every step; the mixed
-// path (mixed.cuh) defers the update outside a 128-column panel to one
+// Small FP64 systems update the whole trailing matrix after every step; large FP64
+// batches (oz_gemm.cuh) defer it outside a 128-column panel to exact INT8 slice
+// products on the tensor cores, and the mixed
+// path (mixed.cuh) to one split-BF16
 // tensor-core product per panel.
 #pragma once
 #include <cooperative_groups.h>
@@ -803,7 +805,7 @@ __device__ __forceinline__ void strip_gemm_body(const BatchT<C2>& b, int k0, int
 //                         block A11 in shared memory (GAUSSZ's unpivoted
 //                         elimination) and inverts the triangles of its 32 x 32
 //                         diagonal blocks (P = inv(L_ii), Q = inv(U_ii));
-//   panel_inv_kernel      W = inv(L11) and V = inv(U11), one CTA each per system;
+//   panel_inv_kernel      W = inv(L11) and V = inv(U11), a CTA per column block;
 //   panel_products_kernel L21 = A21 V for every row below the panel and
 //                         U12 = W A12 for the row strip, in one launch;
 // then the outer update as before.
