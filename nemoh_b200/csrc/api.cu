@@ -1706,10 +1706,7 @@ int nemoh_b200_free_surface(nemoh_ctx* c, double period, int npts, const double*
     const double W = 2. * kPI / period;
     OmegaParams om;
     omega_params(c, W, om, false);
-    // COMPUTE_POTENTIAL_DOMAIN.f90:46 picks the deep-water forms when Depth = 0
-    // or AMH >= 20, AMH being kwave*Depth on the deep-water path of SOLVE_BVP
-    const double amh = om.fd ? om.amh : om.k0 * c->depth;
-    const bool fd = !((c->depth == 0.) || (amh >= 20));
+    const bool fd = field_forms(om, W, c->g, c->depth);
     const size_t ns = (size_t)N * FS_MAXP, nphi = (size_t)npts * FS_MAXP;
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };

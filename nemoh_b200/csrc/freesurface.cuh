@@ -111,6 +111,20 @@ NB_HD __forceinline__ void field_green(const GreenCtx& g, const OmegaParams& om,
   SM2 = (w[0].FS2 + BM * w[1].FS2) * s2;
 }
 
+// The forms of a field point's Green functions at the frequency of om:
+// COMPUTE_POTENTIAL_DOMAIN.f90:46 takes the deep-water ones when Depth = 0 or
+// AMH >= 20, AMH being kwave Depth on the deep-water path of SOLVE_BVP. The
+// root search of the finite-depth path returns an AMH above 20 already for K h
+// from about 16; the deep-water forms' wave number is W^2 / G all the same
+// (VNV, COMPUTE_GREEN_FREESURFACE.f90:199-386), not that root's. Returns true
+// for the finite-depth forms; om.k0 is the forms' wave number.
+inline bool field_forms(OmegaParams& om, double W, double g, double depth) {
+  const double amh = om.fd ? om.amh : om.k0 * depth;
+  const bool fd = !((depth == 0.) || (amh >= 20));
+  if (!fd) om.k0 = W * W / g;
+  return fd;
+}
+
 constexpr int FS_POINTS = 128;
 constexpr int FS_PANELS = 64;   // panels of a CTA: short, so that the grid's last wave is a small part
 constexpr int FS_MAXP = 16;
