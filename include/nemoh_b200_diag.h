@@ -29,6 +29,11 @@ int nemoh_b200_diag_sweep_tuning(long long* keys_tuned, int n, int nsys, int nrh
 /* measured FP64 FMA throughput of a device (TFLOP/s, 2 FLOP per FMA): the
  * best of four launches of independent FMA chains on every SM */
 int nemoh_b200_diag_fp64_peak(int device, double* tflops);
+/* trailing updates of FP64 factorizations that the context has issued on the
+ * tensor cores so far (as launches or into a captured graph; replays of the
+ * graph do not count) */
+struct nemoh_ctx;
+long long nemoh_b200_diag_tensor_updates(const struct nemoh_ctx* ctx);
 /* bounded-wait check of the dataflow sweep: a launch whose only item waits on
  * a ready flag that nothing raises; returns the status word the kernel left
  * (31 = the wait ran out) and the launch's duration */

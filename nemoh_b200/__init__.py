@@ -97,6 +97,8 @@ def load_library():
     L.nemoh_b200_set_graphs.argtypes = [_vp, ctypes.c_int]
     L.nemoh_b200_graph_stats.argtypes = [_vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]
     L.nemoh_b200_solve_requests.argtypes = [_vp, ctypes.c_int, _i, _d, _d, _d]
+    L.nemoh_b200_diag_tensor_updates.argtypes = [_vp]
+    L.nemoh_b200_diag_tensor_updates.restype = ctypes.c_longlong
     L.nemoh_b200_diag_dispersion_root.argtypes = [ctypes.c_double, _d]
     L.nemoh_b200_diag_exponential_fit.argtypes = [ctypes.c_double, ctypes.c_double, _i, _d, _d]
     L.nemoh_b200_diag_theta_quadrature.argtypes = [ctypes.c_double, _d, _d]
@@ -268,6 +270,10 @@ class Solver:
         cap, rep = ctypes.c_longlong(), ctypes.c_longlong()
         load_library().nemoh_b200_graph_stats(self._h, ctypes.byref(cap), ctypes.byref(rep))
         return cap.value, rep.value
+
+    def tensor_updates(self):
+        """Trailing updates of FP64 factorizations issued on the tensor cores so far."""
+        return load_library().nemoh_b200_diag_tensor_updates(self._h)
 
     def set_body_dofs(self, body, dofs):
         """Radiation DOFs (cases.Dof list) of a resident body's serving requests."""

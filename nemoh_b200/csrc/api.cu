@@ -161,6 +161,7 @@ struct nemoh_ctx {
   DevBuf d_froff, d_frord, d_fx, d_fy;   // partial FP64 fallback of a ragged batch
   DevBuf d_flow;                         // workspace of the FP64 dataflow sweep
   OzWork oz;                             // operand images of the FP64 LU's trailing updates
+  long long tensor_updates = 0;          // FP64 trailing updates issued on the tensor cores so far
   long long fallback_systems = 0;         // systems re-solved with FP64 factors so far
   HostBuf h_rag, h_reqs;
   // CUDA graphs of cross-body batches (nemoh_b200_set_graphs)
@@ -519,10 +520,13 @@ void assemble_launch(nemoh_ctx* c, const AsmGroup& ag, const SlotMesh* dmesh) {
 }
 
 // The systems of a batch: nsys systems of order n (uniform, the current mesh),
-// or of orders up to n described by rg (ragged, several bodies).
+// or of orders up to n described by rg (ragged, several bodies). images: the
+// context holds the operand images of their FP64 updates (fp64_images, once per
+// batch and before a launch sequence that may be captured).
 struct Shape {
   int n;
   Ragged rg;
+  bool images = false;
 };
 Shape uniform_shape(const nemoh_ctx* c) { return Shape{c->nfa, Ragged()}; }
 
@@ -532,19 +536,19 @@ Batch dbatch(nemoh_ctx* c, const Shape& sh) {
 }
 
 // Operand images of the FP64 LU's tensor-core updates (oz_gemm.cuh) for nsys
-// systems of order up to n; false where there is no trailing update or no room
-// for them (the FP64 fallback of a mixed batch that fills the device): the
+// systems of order up to sh.n; false where there is no trailing update or no
+// room for them (the FP64 fallback of a mixed batch that fills the device): the
 // update then runs on the FP64 pipe.
-bool fp64_images(nemoh_ctx* c, int nsys, int n) {
-  const double rest = n - LU_OUTER;
+bool fp64_images(nemoh_ctx* c, int nsys, const Shape& sh) {
+  const double rest = sh.n - LU_OUTER;
   if (!tc_enabled() || rest <= 0 || rest * rest * nsys < OZ_MIN_ENTRIES) return false;
-  return c->oz.ensure(nsys, n) == cudaSuccess;
+  return c->oz.ensure(nsys, sh.n) == cudaSuccess;
 }
 
 void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
   Batch b = dbatch(c, sh);
   const int N = sh.n;
-  const bool images = fp64_images(c, nsys, N);
+  const bool images = sh.images;
   // Panel pairs are merged where the update fills the device: after the first
   // panel only the next panel's columns and rows are updated, the rest of the
   // trailing matrix takes both panels' products in the next panel's update, so
@@ -570,6 +574,7 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
         const OzStride st = oz_stride(c->oz);
         const OzSet cur = oz_set(c->oz, set, s0);
         int* status = c->d_status.as<int>();
+        ++c->tensor_updates;
         oz_prep(cur, st, bg, k0, ns, sg, c->launches);
         if (late) {
           oz_apply(cur, oz_set(c->oz, set ^ 1, s0), st, bg, k0, ns, sg, c->launches, status, false);
@@ -612,11 +617,12 @@ void trsm_fp64(nemoh_ctx* c, int nsys, int nrhs, const Shape& sh) {
 // factored again in FP64 on the device and solved from the original
 // right-hand sides, which the refinement kept in mixed.b. d_D then holds the
 // FP64 factors (lu64) instead of the matrix.
-void mixed_fallback(nemoh_ctx* c, int nsys, int nrhs, const Shape& sh) {
+void mixed_fallback(nemoh_ctx* c, int nsys, int nrhs, Shape sh) {
   MixedWork& w = c->mixed;
   const size_t N = sh.n;
   CK(c->d_inv.ensure((size_t)nsys * ((N + TB - 1) / TB) * 2 * TB * TB * sizeof(double2)));
   CK(cudaMemcpyAsync(c->d_X.p, w.b, (size_t)nsys * N * nrhs * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
+  sh.images = fp64_images(c, nsys, sh);
   factor_fp64(c, nsys, sh);
   trsm_fp64(c, nsys, nrhs, sh);
   c->lu64 = true;
@@ -670,7 +676,8 @@ void mixed_fallback_ragged(nemoh_ctx* c, int nsys, int nrhs, const Shape& sh) {
   for (int j = 0; j < nf; ++j)   // a system's right-hand sides: ord x nrhs, contiguous
     CK(cudaMemcpyAsync(fx + j * xf, w.b + bad[j] * xs, (size_t)ord_f[j] * nrhs * sizeof(double2),
                        cudaMemcpyDeviceToDevice, c->stream));
-  const Shape shf{ord_f[0], Ragged{c->d_froff.as<long long>(), c->d_frord.as<int>(), ord_f.data(), off_f.data()}};
+  Shape shf{ord_f[0], Ragged{c->d_froff.as<long long>(), c->d_frord.as<int>(), ord_f.data(), off_f.data()}};
+  shf.images = fp64_images(c, nf, shf);
   factor_fp64(c, nf, shf);
   const SweepSync sync = fp64_sync(c, nf, shf.n);
   CK(trsm_sweep_tuned<double2>(dbatch(c, shf), c->d_inv.as<double2>(), fx, c->d_fy.as<double2>(), nf, nrhs,
@@ -695,7 +702,7 @@ void mixed_solve(nemoh_ctx* c, int nsys, int nrhs, const Shape& sh) {
 
 // pre (mixed precision, uniform batches): systems [0, pre) were factored on
 // stream2, whose event ev_pipe[1] the refinement waits for
-void factor_and_solve(nemoh_ctx* c, int nsys, int nrhs, bool have_rhs, const Shape& sh, int pre = 0) {
+void factor_and_solve(nemoh_ctx* c, int nsys, int nrhs, bool have_rhs, Shape sh, int pre = 0) {
   c->lu64 = c->mode == NEMOH_B200_FP64;
   CK(cudaEventRecord(c->ev_lu[0], c->stream));
   if (c->mode == NEMOH_B200_MIXED) {
@@ -706,6 +713,7 @@ void factor_and_solve(nemoh_ctx* c, int nsys, int nrhs, bool have_rhs, const Sha
     CK(cudaEventRecord(c->ev_lu[1], c->stream));
     if (have_rhs) mixed_solve(c, nsys, nrhs, sh);
   } else {
+    if (!sh.rg.host_off) sh.images = fp64_images(c, nsys, sh);   // a ragged batch has them with its buffers
     factor_fp64(c, nsys, sh);
     CK(cudaEventRecord(c->ev_lu[1], c->stream));
     if (have_rhs) trsm_fp64(c, nsys, nrhs, sh);
@@ -908,7 +916,8 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   c->cap_nfa = -1;
   c->w_previous = -1.;
   const long long xs = (long long)N * nrhs;
-  const Shape sh{nmax, Ragged{c->d_roff.as<long long>(), c->d_rord.as<int>(), ord.data(), off.data()}};
+  Shape sh{nmax, Ragged{c->d_roff.as<long long>(), c->d_rord.as<int>(), ord.data(), off.data()}};
+  if (c->mode == NEMOH_B200_FP64) sh.images = fp64_images(c, nsys, sh);
   OmegaParams* hom = c->h_oms.as<OmegaParams>();
   auto host_setup = [&](int j) {
     BodyState& b = *c->bodies[body[items[j]]];
@@ -969,11 +978,7 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   const bool mixed = c->mode == NEMOH_B200_MIXED;
   const int max_it = refine_max_it(), passes = mixed ? std::min(REFINE_CHUNK, max_it) : 0;
   // the FP64 sweeps' workspace grows here, never inside a captured sequence
-  // (nor the operand images of its trailing updates)
-  if (!mixed) {
-    fp64_sync(c, nsys, nmax);
-    fp64_images(c, nsys, nmax);
-  }
+  if (!mixed) fp64_sync(c, nsys, nmax);
   // a captured sequence holds every buffer address it was captured with: the
   // key covers them all, so a buffer that moved since is captured again
   std::vector<long long> sig = {c->mode, nrhs, k, nsys, nmax, nint_max, passes, (long long)nvel_d,
@@ -986,7 +991,8 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
                                 (long long)c->mixed.inv, (long long)c->mixed.pinv, (long long)c->mixed.norms,
                                 (long long)c->mixed.state, (long long)c->mixed.tc.a, (long long)c->mixed.tc.b,
                                 (long long)c->mixed.tc.wv, (long long)c->mixed.flow, (long long)c->mixed.act,
-                                (long long)c->d_flow.p, (long long)c->oz.a, (long long)c->oz.b, (long long)c->oz.sc};
+                                (long long)c->d_flow.p, (long long)c->oz.a, (long long)c->oz.b, (long long)c->oz.sc,
+                                (long long)sh.images};
   for (const AsmGroup& g : groups)
     sig.insert(sig.end(), {g.ninfd, g.nfd, g.n_infd, g.n_fd, (long long)g.slot_rk_infd, (long long)g.slot_rk_fd});
   sig.insert(sig.end(), ord.begin(), ord.end());
@@ -2032,6 +2038,8 @@ int nemoh_b200_diag_fp64_peak(int device, double* tflops) {
 // blocks) with the item counter started past level 0, so the level-1 item
 // waits on a ready flag that no item raises. The wait runs out, records
 // ST_SWEEP_TIMEOUT and the launch returns; the device stays usable.
+long long nemoh_b200_diag_tensor_updates(const nemoh_ctx* c) { return c ? c->tensor_updates : 0; }
+
 int nemoh_b200_diag_sweep_timeout(int device, int* status, double* ms) {
   if (!status || !ms) return NEMOH_B200_EINVAL;
   return guarded(nullptr, [&] {

@@ -188,15 +188,16 @@ struct OzWork {
     have_a = have_b = have_sc = 0;
   }
   ~OzWork() { release(); }
+  // all of the images or none of them
   cudaError_t ensure(int ns, int n, bool headroom = false) {
     tiles = (n + OZ_M - 1) / OZ_M;
     nsys = ns;
     const size_t t = 2 * (size_t)ns * tiles;
     cudaError_t e = grow_alloc(reinterpret_cast<void**>(&a), &have_a, t * OZ_NCH * OZ_S * OZ_A, headroom);
-    if (e) return e;
-    e = grow_alloc(reinterpret_cast<void**>(&b), &have_b, t * 2 * OZ_NCH * OZ_S * OZ_B, headroom);
-    if (e) return e;
-    return grow_alloc(reinterpret_cast<void**>(&sc), &have_sc, t * 2 * OZ_M * sizeof(double), headroom);
+    if (!e) e = grow_alloc(reinterpret_cast<void**>(&b), &have_b, t * 2 * OZ_NCH * OZ_S * OZ_B, headroom);
+    if (!e) e = grow_alloc(reinterpret_cast<void**>(&sc), &have_sc, t * 2 * OZ_M * sizeof(double), headroom);
+    if (e) release();
+    return e;
   }
 };
 inline size_t oz_bytes_per_system(size_t n) {

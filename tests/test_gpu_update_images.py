@@ -1,0 +1,89 @@
+"""Operand images of the FP64 LU's tensor-core updates when device memory is
+short: they are had for a whole batch before anything of it is launched, or the
+update runs on the FP64 pipe, also in batches that are captured into graphs;
+what a shortage leaves allocated is given back. Memory is made short by
+allocating the rest of the device."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import nemoh_b200 as nb
+from nemoh_b200 import cases as C
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+def _hull(n):
+    """A hull of exactly n panels: a cylinder whose wall and bottom are cut to the count."""
+    f = max(1.0, np.sqrt(n / 300.0))
+    m = C.cylinder_mesh(6.0, 12.0, 2 * round(12 * f), round(10 * f) + 1, round(5 * f), 2 * round(6 * f) + 2)
+    return C.Mesh(m.nodes, m.panels[-n:], 0)
+
+
+def _body(n):
+    return C.Case(_hull(n), np.array([0.8]), np.array([0.0]), C.six_dofs(), C.six_dofs(), depth=0.0)
+
+
+def _items(rng, n, count):
+    nv = rng.standard_normal((count, n, 2)) + 1j * rng.standard_normal((count, n, 2))
+    return np.linspace(0.5, 1.2, count), [np.asfortranarray(v) for v in nv]
+
+
+def _free():
+    import torch
+    return torch.cuda.mem_get_info(0)[0]
+
+
+@contextlib.contextmanager
+def _only(room):
+    """All of the device but `room` bytes allocated."""
+    import torch
+    held = []
+    try:
+        for size in (1 << 33, 1 << 30, 1 << 27, 1 << 24, 1 << 22):
+            while _free() > room + size:
+                try:
+                    held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+                except torch.OutOfMemoryError:
+                    break
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("room", [20 * MB, 60 * MB])   # none of the images fits; the first of them does
+def test_captured_batch_without_room_for_images(room):
+    rng = np.random.default_rng(1)
+    n, count = 400, 21
+    om, nv = _items(rng, n, count)
+    om_a, nv_a = _items(rng, 200, 200)
+    with nb.Solver(0, nb.FP64) as s:
+        s.add_body(_body(n))
+        ref = s.solve_bodies(np.zeros(count, np.int32), om, nv)
+        assert s.tensor_updates() > 0   # with room the batch takes them
+    with nb.Solver(0, nb.FP64) as s:
+        s.add_body(_body(n))
+        s.add_body(_body(200))
+        s.prepare_bodies()
+        s.set_graphs(True)
+        # a batch of many small systems provides every other buffer
+        for _ in range(2):
+            s.solve_bodies(np.ones(200, np.int32), om_a, nv_a)
+        assert s.tensor_updates() == 0
+        captures, replays = s.graph_stats()
+        with _only(room):
+            before = _free()
+            runs = [s.solve_bodies(np.zeros(count, np.int32), om, nv) for _ in range(4)]
+            after = _free()
+        assert s.tensor_updates() == 0
+        assert s.graph_stats() == (captures + 1, replays + 2)
+        assert before - after < 16 * MB   # no part of the images is kept
+        runs.append(s.solve_bodies(np.zeros(count, np.int32), om, nv))   # with room again
+        assert s.tensor_updates() > 0
+    for got in runs:
+        for g, r in zip(got, ref):
+            # both are backward-stable solves of well-conditioned systems
+            assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
