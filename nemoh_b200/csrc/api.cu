@@ -539,10 +539,10 @@ Batch dbatch(nemoh_ctx* c, const Shape& sh) {
 // systems of order up to sh.n; false where there is no trailing update or no
 // room for them (the FP64 fallback of a mixed batch that fills the device): the
 // update then runs on the FP64 pipe.
-bool fp64_images(nemoh_ctx* c, int nsys, const Shape& sh) {
+bool fp64_images(nemoh_ctx* c, int nsys, const Shape& sh, bool headroom = false) {
   const double rest = sh.n - LU_OUTER;
   if (!tc_enabled() || rest <= 0 || rest * rest * nsys < OZ_MIN_ENTRIES) return false;
-  return c->oz.ensure(nsys, sh.n) == cudaSuccess;
+  return c->oz.ensure(nsys, sh.n, headroom) == cudaSuccess;
 }
 
 void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
@@ -917,7 +917,7 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   c->w_previous = -1.;
   const long long xs = (long long)N * nrhs;
   Shape sh{nmax, Ragged{c->d_roff.as<long long>(), c->d_rord.as<int>(), ord.data(), off.data()}};
-  if (c->mode == NEMOH_B200_FP64) sh.images = fp64_images(c, nsys, sh);
+  if (c->mode == NEMOH_B200_FP64) sh.images = fp64_images(c, nsys, sh, headroom);
   OmegaParams* hom = c->h_oms.as<OmegaParams>();
   auto host_setup = [&](int j) {
     BodyState& b = *c->bodies[body[items[j]]];

@@ -87,3 +87,19 @@ def test_captured_batch_without_room_for_images(room):
         for g, r in zip(got, ref):
             # both are backward-stable solves of well-conditioned systems
             assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
+
+
+def test_ragged_images_grow_with_headroom():
+    """A stream of batches that each need a little more reallocates the images
+    rarely (a reallocation synchronises the device), as its other buffers."""
+    rng = np.random.default_rng(2)
+    with nb.Solver(0, nb.FP64) as s:
+        s.add_body(_body(400))
+        s.prepare_bodies()
+        free = []
+        for count in range(40, 48):   # images of 192 to 226 MB
+            om, nv = _items(rng, 400, count)
+            s.solve_bodies(np.zeros(count, np.int32), om, nv)
+            free.append(_free())
+        assert s.tensor_updates() > 0
+    assert len(set(free)) == 1, free
