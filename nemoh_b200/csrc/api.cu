@@ -344,6 +344,8 @@ void upload_geometry(nemoh_ctx* c, int np, int nfa, int nsymy, const double* xyz
 int batch_capacity(nemoh_ctx* c, int nrhs, int want) {
   if (want <= c->cap_slots && nrhs <= c->cap_nrhs && c->nfa == c->cap_nfa && ncls(c) == c->cap_cls)
     return want;   // buffers already fit (same mesh size as the last batch)
+  // a mixed batch grows into the room of an earlier FP64 fallback's images
+  if (c->mode == NEMOH_B200_MIXED) c->oz.release();
   size_t fr = 0, tot = 0;
   CK(cudaMemGetInfo(&fr, &tot));
   const size_t N = c->nfa, cls = ncls(c);
@@ -1132,11 +1134,23 @@ void solve_bodies_impl(nemoh_ctx* c, int nitem, const int* body, const double* o
   CK(cudaEventRecord(rk1.e, c->stream));
   // admission by HBM footprint: 80% of the free memory, the batch's own
   // buffers counted as free
-  size_t fr = 0, tot = 0;
-  CK(cudaMemGetInfo(&fr, &tot));
-  const size_t have = c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes + c->d_diag.bytes +
-                      c->mixed.bytes() + c->oz.bytes();
-  size_t budget = (size_t)((fr + have) * 0.8);
+  auto free_bytes = [&] {
+    size_t fr = 0, tot = 0;
+    CK(cudaMemGetInfo(&fr, &tot));
+    // the FP64 updates' images are a mixed batch's only while it falls back
+    const size_t images = c->mode == NEMOH_B200_FP64 ? c->oz.bytes() : 0;
+    return (size_t)((fr + c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes +
+                     c->d_diag.bytes + c->mixed.bytes() + images) * 0.8);
+  };
+  size_t budget = free_bytes();
+  if (c->mode == NEMOH_B200_MIXED && c->oz.bytes()) {   // an earlier fallback's: given back where the call needs the room
+    size_t need = 0;
+    for (int i : idx) need += item_bytes(c, *c->bodies[body[i]], c->bodies[body[idx[0]]]->nfa, nrhs);
+    if (need > budget) {
+      c->oz.release();
+      budget = free_bytes();
+    }
+  }
   // NEMOH_B200_BATCH_BYTES lowers the budget (tests use it to split a call
   // into several batches)
   if (const char* e = std::getenv("NEMOH_B200_BATCH_BYTES")) {

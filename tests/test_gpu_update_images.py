@@ -1,8 +1,9 @@
 """Operand images of the FP64 LU's tensor-core updates when device memory is
 short: they are had for a whole batch before anything of it is launched, or the
 update runs on the FP64 pipe, also in batches that are captured into graphs;
-what a shortage leaves allocated is given back. Memory is made short by
-allocating the rest of the device."""
+what a shortage leaves allocated is given back; and a mixed-precision context,
+in which only the FP64 fallback takes images, doesn't count them as room for
+its batches. Memory is made short by allocating the rest of the device."""
 import contextlib
 
 import numpy as np
@@ -103,3 +104,37 @@ def test_ragged_images_grow_with_headroom():
             free.append(_free())
         assert s.tensor_updates() > 0
     assert len(set(free)) == 1, free
+
+
+@pytest.mark.parametrize("ragged", [False, True])
+def test_mixed_batches_after_a_fallback_in_short_memory(ragged, monkeypatch):
+    """The fallback of 40 systems leaves images of 183 MB; with 100 MB free a
+    larger mixed call is solved, in as many batches as fit."""
+    rng = np.random.default_rng(3)
+    n = 400
+    case = _body(n)
+    nds = C.generalised_normals(case)
+    om, nv = _items(rng, n, 72)
+
+    def solve(s, count):
+        if ragged:
+            return np.stack(s.solve_bodies(np.zeros(count, np.int32), om[:count], nv[:count]), axis=2)
+        return s.solve_frequencies(om[:count], np.asfortranarray(np.stack(nv[:count], axis=2)), nds)
+
+    with nb.Solver(0, nb.MIXED) as s:
+        s.add_body(case)
+        s.set_case(case)
+        ref = solve(s, 72)
+    with nb.Solver(0, nb.MIXED) as s:
+        s.add_body(case)
+        s.set_case(case)
+        s.prepare_bodies()
+        monkeypatch.setenv("NEMOH_B200_REFINE_MAX_IT", "1")
+        solve(s, 40)
+        monkeypatch.delenv("NEMOH_B200_REFINE_MAX_IT")
+        assert s.tensor_updates() > 0
+        with _only(100 * MB):
+            for count in (44, 48, 52, 56, 60, 64, 68, 72):
+                got = solve(s, count)
+                # refined to 1e-12 of the right-hand side on either side
+                assert np.abs(got - ref[:, :, :count]).max() <= 1e-10 * np.abs(ref).max()
