@@ -532,6 +532,16 @@ struct Shape {
 };
 Shape uniform_shape(const nemoh_ctx* c) { return Shape{c->nfa, Ragged()}; }
 
+// sum of f(order - k) over the batch's systems that reach beyond column k (a
+// ragged batch's orders decrease)
+template <class F>
+double trailing_sum(const Shape& sh, int nsys, int k, F f) {
+  if (!sh.rg.host_ord) return k < sh.n ? nsys * (double)f(sh.n - k) : 0.;
+  double t = 0.;
+  for (int s = 0; s < nsys && sh.rg.host_ord[s] > k; ++s) t += f(sh.rg.host_ord[s] - k);
+  return t;
+}
+
 Batch dbatch(nemoh_ctx* c, const Shape& sh) {
   // FP64 keeps the per-step row-strip updates (FP64 GEMM tiles beat the fused strip solve there)
   return make_batch<double2>(c->d_D.as<double2>(), sh.n, c->d_diag.as<double2>(), nullptr, sh.rg);
@@ -542,8 +552,8 @@ Batch dbatch(nemoh_ctx* c, const Shape& sh) {
 // room for them (the FP64 fallback of a mixed batch that fills the device): the
 // update then runs on the FP64 pipe.
 bool fp64_images(nemoh_ctx* c, int nsys, const Shape& sh, bool headroom = false) {
-  const double rest = sh.n - LU_OUTER;
-  if (!tc_enabled() || rest <= 0 || rest * rest * nsys < OZ_MIN_ENTRIES) return false;
+  if (!tc_enabled() || trailing_sum(sh, nsys, LU_OUTER, [](double rest) { return rest * rest; }) < OZ_MIN_ENTRIES)
+    return false;
   return c->oz.ensure(nsys, sh.n, headroom) == cudaSuccess;
 }
 
@@ -566,8 +576,7 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
       b, nsys, c->d_status.as<int>(), c->stream, c->launches,
       [&](Batch bg, int ns, cudaStream_t sg, int s0, int k0, int kend) {
         bool& late = deferred[s0];
-        const double rest = bg.n - kend;
-        if (!images || !(late || rest * rest * nsys >= OZ_MIN_ENTRIES)) {
+        if (!images || !(late || trailing_sum(sh, nsys, kend, [](double rest) { return rest * rest; }) >= OZ_MIN_ENTRIES)) {
           zgemm_update<double2>(bg, k0, kend - k0, Rect{kend, bg.n, kend, bg.n}, ns, sg);
           ++c->launches;
           return;
@@ -582,7 +591,7 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
           oz_apply(cur, oz_set(c->oz, set ^ 1, s0), st, bg, k0, ns, sg, c->launches, status, false);
           late = false;
         } else {
-          late = kend + LU_OUTER < bg.n && oz_tiles((int)rest, nsys) >= OZ_MERGE_TILES;
+          late = kend + LU_OUTER < bg.n && trailing_sum(sh, nsys, kend, oz_tiles) >= OZ_MERGE_TILES;
           oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, late);
         }
       },
@@ -843,7 +852,7 @@ size_t item_bytes(const nemoh_ctx* c, const BodyState& b, int nmax, int nrhs) {
     mats += n * n * sizeof(float2);
     per_sys += nm * nrhs * (2 * sizeof(double2) + 2 * sizeof(float2)) + (DIAG_SCRATCH + PINV_SCRATCH) * sizeof(float2) +
                nblk * 2 * TB * TB * sizeof(float2) + tc_bytes_per_system(nm);
-  } else {
+  } else if (nm > LU_OUTER) {
     per_sys += oz_bytes_per_system(nm);
   }
   return cls * (mats + per_sys) + sizeof(OmegaParams) + sizeof(SlotMesh) + sizeof(ItemDesc);

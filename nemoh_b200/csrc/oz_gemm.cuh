@@ -57,15 +57,15 @@ constexpr int OZ_EC = OZ_N / (OZ_EPI_WARPS / 4);   // complex columns per epilog
 constexpr int OZ_BATCH = 2;                        // of them loaded at once
 constexpr int OZ_SMEM = OZ_SLOTS * OZ_SLOT + 256 + 2 * 2 * OZ_N * (int)sizeof(double);
 constexpr int OZ_EMIN = -250;                    // smallest scale exponent (rows and columns below it are round-off)
-// Trailing entries of a batch (over its systems) from which an update takes this
-// path; below it the FP64 pipe's one launch is as fast as the images and the
+// Trailing entries of a batch (summed over its systems that the panel has not
+// finished) from which an update takes this path; below it the FP64 pipe's one launch is as fast as the images and the
 // update, which then cover few SMs. LU in ms, FP64 pipe against this path: 10
 // systems of 420 panels (0.9 M entries) 0.71 / 0.71, 4 of 588 (0.8 M) 0.94 / 0.95,
 // 2 of 894 (1.2 M) 1.08 / 1.08, 4 of 894 (2.3 M) 1.32 / 1.22, 2 of 1,430 (3.4 M)
 // 2.24 / 1.99, 20 of 588 (4.2 M) 1.44 / 1.25, 1 of 2,380 (5.1 M) 4.21 / 3.37, 20 of
 // 2,380 (101 M) 37.0 / 17.2.
 constexpr double OZ_MIN_ENTRIES = 1.5e6;
-// Tiles of a full update from which panel pairs are merged (four per SM): the
+// Tiles of a full update (summed likewise) from which panel pairs are merged (four per SM): the
 // merged form reads and writes the trailing block once per pair, the corner
 // update it needs is a launch of one tile's latency more. LU in ms, never merged /
 // merged from 148 tiles / from 600: 20 systems of 420 0.77 / 0.81 / 0.78, 10 of 894
@@ -754,9 +754,9 @@ inline void oz_prep(const OzSet& s, const OzStride& st, Batch b, int k0, int nsy
   ++launches;
 }
 
-// tiles of a full update of the trailing block
-inline long long oz_tiles(int rest, int nsys) {
-  return (long long)((rest + OZ_M - 1) / OZ_M) * ((rest + OZ_N - 1) / OZ_N) * nsys;
+// tiles of a full update of one system's trailing block
+inline long long oz_tiles(int rest) {
+  return (long long)((rest + OZ_M - 1) / OZ_M) * ((rest + OZ_N - 1) / OZ_N);
 }
 
 // The panel's trailing block from its images (and the deferred panel's in prev);
@@ -775,7 +775,7 @@ inline void oz_apply(const OzSet& cur, const OzSet& prev, const OzStride& st, Ba
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   });
-  const long long tiles = corner ? (long long)(CW * nti + std::max(0, ntc - CW)) * nsys : oz_tiles(rest, nsys);
+  const long long tiles = corner ? (long long)(CW * nti + std::max(0, ntc - CW)) * nsys : oz_tiles(rest) * nsys;
   const int grid = (int)std::min<long long>(tiles, sms > 0 ? sms : 148);
   oz_update_kernel<<<grid, OZ_THREADS, OZ_SMEM, stream>>>(b, k0, cur, prev, st, nsys, status, nti, ntc, corner ? 1 : 0);
   ++launches;

@@ -138,3 +138,44 @@ def test_mixed_batches_after_a_fallback_in_short_memory(ragged, monkeypatch):
                 got = solve(s, count)
                 # refined to 1e-12 of the right-hand side on either side
                 assert np.abs(got - ref[:, :, :count]).max() <= 1e-10 * np.abs(ref).max()
+
+
+def _ragged(s, ids, counts):
+    rng = np.random.default_rng(4)
+    bodies, nv = [], []
+    for b, (n, count) in zip(ids, counts):
+        bodies += [b] * count
+        nv += _items(rng, n, count)[1]
+    s.solve_bodies(np.array(bodies, np.int32), np.linspace(0.5, 1.2, len(bodies)), nv)
+
+
+@pytest.mark.parametrize("counts,updates", [
+    ([(700, 1), (200, 40)], (0, 0)),     # 0.54 M trailing entries after the first panel, in 41 systems
+    ([(1100, 2), (200, 20)], (1, 4)),    # 1.99 M after the first panel (an update per stream group), 1.42 M after it
+    ([(1100, 4), (300, 4)], (3, 10)),    # 3.9, 2.9, 2.1 and 1.4 M: three panels
+])
+def test_ragged_batches_count_the_systems_that_go_on(counts, updates):
+    """The tensor-core update is for batches of 1.5 M trailing entries, counted
+    over the systems that have some."""
+    with nb.Solver(0, nb.FP64) as s:
+        ids = [s.add_body(_body(n)) for n, _ in counts]
+        _ragged(s, ids, counts)
+        assert updates[0] <= s.tensor_updates() <= updates[1]
+
+
+def test_small_systems_are_not_charged_for_images(monkeypatch):
+    """64 items of 100 panels (about 0.7 MB each) fit a budget of 64 MB in one
+    batch: systems of one panel have no trailing update and no images."""
+    om, nv = _items(np.random.default_rng(5), 100, 64)
+
+    def launches(s):
+        before = s.launches
+        s.solve_bodies(np.zeros(64, np.int32), om, nv)
+        return s.launches - before
+
+    with nb.Solver(0, nb.FP64) as s:
+        s.add_body(_body(100))
+        s.prepare_bodies()
+        whole = launches(s)
+        monkeypatch.setenv("NEMOH_B200_BATCH_BYTES", str(64 * MB))
+        assert launches(s) == whole
