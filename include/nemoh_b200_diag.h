@@ -34,6 +34,13 @@ int nemoh_b200_diag_fp64_peak(int device, double* tflops);
  * graph do not count) */
 struct nemoh_ctx;
 long long nemoh_b200_diag_tensor_updates(const struct nemoh_ctx* ctx);
+/* the tensor-core trailing update by itself, on host matrices: `nsys` complex
+ * column-major matrices n * n elements apart, of order n (orders null) or
+ * orders[s] <= n, decreasing, orders[0] = n (leading dimension orders[s]).
+ * panels 1: A22 -= A21 A12 with the first 128 columns and rows as they are. 2: that
+ * update for the next 128 columns and rows only, then both panels' products (the
+ * second panel's operands as the first update left them) into the rest. */
+int nemoh_b200_diag_fp64_update(int device, int n, int nsys, const int* orders, int panels, double* a);
 /* bounded-wait check of the dataflow sweep: a launch whose only item waits on
  * a ready flag that nothing raises; returns the status word the kernel left
  * (31 = the wait ran out) and the launch's duration */

@@ -102,6 +102,7 @@ struct BodyState {
   int nq_state = 0;
   int ndof = 0;   // radiation DOFs of serving requests (nemoh_b200_set_body_dofs)
   DevBuf d_xyz, d_m, d_rec, d_rows, d_nds, d_dofs;
+  std::vector<char> wide;   // oz_wide of the mesh
   // frequency-independent Rankine part per depth regime (0 deep water, 1
   // finite depth), kept with the resident body once evaluated
   DevBuf rk[2];
@@ -131,6 +132,7 @@ struct nemoh_ctx {
   double rho = 0, g = 0, depth = 0, zer = 0, gm = 0;
   double ro_eps2 = 0;   // largest x with sqrt(x) <= 1e-4
   DevBuf d_xyz, d_m, d_rec, d_rows;
+  std::vector<char> wide;   // oz_wide of the mesh
   // per-call workspace
   DevBuf d_D, d_S, d_X, d_Y, d_diag, d_inv, d_oms, d_slots, d_nvel, d_nds, d_force, d_kochin, d_pre, d_fs, d_irf;
   HostBuf h_oms, h_slots;
@@ -308,7 +310,7 @@ void omega_params_env(const Env& env, double W, OmegaParams& om, bool advance_nq
 // (PREPARE_MESH.f90:58-69: the largest pairwise |dx| is max - min), GM by a
 // device reduction. Synchronises the context's stream.
 void upload_geometry(nemoh_ctx* c, int np, int nfa, int nsymy, const double* xyz, const int* m1234, DevBuf& d_xyz,
-                     DevBuf& d_m, DevBuf& d_rec, DevBuf& d_rows, double& zer, double& gm) {
+                     DevBuf& d_m, DevBuf& d_rec, DevBuf& d_rows, double& zer, double& gm, std::vector<char>& wide) {
   for (int i = 0; i < 4 * nfa; ++i)
     if (m1234[i] < 1 || m1234[i] > np) throw Fail{NEMOH_B200_EINVAL, "panel node index out of range"};
   double xmin = xyz[0], xmax = xyz[0], ymin = xyz[1], ymax = xyz[1], yabs = 0;
@@ -322,6 +324,7 @@ void upload_geometry(nemoh_ctx* c, int np, int nfa, int nsymy, const double* xyz
   const double GL0 = xmax - xmin;
   const double BL = nsymy ? 2. * yabs : ymax - ymin;
   zer = -1.E-5 * std::max(GL0, BL);
+  wide = oz_wide(nfa, xyz, m1234);
   CK(d_xyz.ensure(sizeof(double) * 3 * np));
   CK(d_m.ensure(sizeof(int) * 4 * nfa));
   CK(d_rec.ensure(sizeof(PanelRec) * nfa));
@@ -524,13 +527,16 @@ void assemble_launch(nemoh_ctx* c, const AsmGroup& ag, const SlotMesh* dmesh) {
 // The systems of a batch: nsys systems of order n (uniform, the current mesh),
 // or of orders up to n described by rg (ragged, several bodies). images: the
 // context holds the operand images of their FP64 updates (fp64_images, once per
-// batch and before a launch sequence that may be captured).
+// batch and before a launch sequence that may be captured). wide: the panels whose
+// updates stay on the FP64 pipe (oz_wide, for any of the systems).
 struct Shape {
   int n;
   Ragged rg;
+  std::vector<char> wide;
   bool images = false;
+  bool wide_panel(int k0) const { return k0 / LU_OUTER < (int)wide.size() && wide[k0 / LU_OUTER]; }
 };
-Shape uniform_shape(const nemoh_ctx* c) { return Shape{c->nfa, Ragged()}; }
+Shape uniform_shape(const nemoh_ctx* c) { return Shape{c->nfa, Ragged(), c->wide}; }
 
 // sum of f(order - k) over the batch's systems that reach beyond column k (a
 // ragged batch's orders decrease)
@@ -554,6 +560,9 @@ Batch dbatch(nemoh_ctx* c, const Shape& sh) {
 bool fp64_images(nemoh_ctx* c, int nsys, const Shape& sh, bool headroom = false) {
   if (!tc_enabled() || trailing_sum(sh, nsys, LU_OUTER, [](double rest) { return rest * rest; }) < OZ_MIN_ENTRIES)
     return false;
+  bool any = false;
+  for (int k0 = 0; k0 + LU_OUTER < sh.n; k0 += LU_OUTER) any |= !sh.wide_panel(k0);
+  if (!any) return false;
   return c->oz.ensure(nsys, sh.n, headroom) == cudaSuccess;
 }
 
@@ -576,7 +585,10 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
       b, nsys, c->d_status.as<int>(), c->stream, c->launches,
       [&](Batch bg, int ns, cudaStream_t sg, int s0, int k0, int kend) {
         bool& late = deferred[s0];
-        if (!images || !(late || trailing_sum(sh, nsys, kend, [](double rest) { return rest * rest; }) >= OZ_MIN_ENTRIES)) {
+        const bool tensor =
+            late || (images && !sh.wide_panel(k0) &&
+                     trailing_sum(sh, nsys, kend, [](double rest) { return rest * rest; }) >= OZ_MIN_ENTRIES);
+        if (!tensor) {
           zgemm_update<double2>(bg, k0, kend - k0, Rect{kend, bg.n, kend, bg.n}, ns, sg);
           ++c->launches;
           return;
@@ -591,7 +603,8 @@ void factor_fp64(nemoh_ctx* c, int nsys, const Shape& sh) {
           oz_apply(cur, oz_set(c->oz, set ^ 1, s0), st, bg, k0, ns, sg, c->launches, status, false);
           late = false;
         } else {
-          late = kend + LU_OUTER < bg.n && trailing_sum(sh, nsys, kend, oz_tiles) >= OZ_MERGE_TILES;
+          late = kend + LU_OUTER < bg.n && !sh.wide_panel(kend) &&
+                 trailing_sum(sh, nsys, kend, oz_tiles) >= OZ_MERGE_TILES;
           oz_apply(cur, OzSet(), st, bg, k0, ns, sg, c->launches, status, late);
         }
       },
@@ -687,7 +700,7 @@ void mixed_fallback_ragged(nemoh_ctx* c, int nsys, int nrhs, const Shape& sh) {
   for (int j = 0; j < nf; ++j)   // a system's right-hand sides: ord x nrhs, contiguous
     CK(cudaMemcpyAsync(fx + j * xf, w.b + bad[j] * xs, (size_t)ord_f[j] * nrhs * sizeof(double2),
                        cudaMemcpyDeviceToDevice, c->stream));
-  Shape shf{ord_f[0], Ragged{c->d_froff.as<long long>(), c->d_frord.as<int>(), ord_f.data(), off_f.data()}};
+  Shape shf{ord_f[0], Ragged{c->d_froff.as<long long>(), c->d_frord.as<int>(), ord_f.data(), off_f.data()}, sh.wide};
   shf.images = fp64_images(c, nf, shf);
   factor_fp64(c, nf, shf);
   const SweepSync sync = fp64_sync(c, nf, shf.n);
@@ -868,11 +881,13 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   std::vector<char> has_rk(k);
   std::vector<SlotMesh> sm(k);
   std::vector<ItemDesc> it(k);
+  std::vector<char> wide(c->bodies[body[items[0]]]->wide.size());
   long long mat = 0;
   int nint_max = 0;
   for (int j = 0; j < k; ++j) {
     const int i = items[j];
     const BodyState& b = *c->bodies[body[i]];
+    for (size_t q = 0; q < b.wide.size(); ++q) wide[q] |= b.wide[q];
     const bool fd = finite_depth(Env{b.g, b.depth, b.gm, nullptr}, 2. * kPI / (2. * kPI / omegas[i]));
     has_rk[j] = b.rk_valid[fd];
     sm[j] = SlotMesh{b.d_rec.as<PanelRec>(), b.d_rows.as<double>(), mat, b.nfa, b.nsymy, b.zer,
@@ -927,7 +942,7 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   c->cap_nfa = -1;
   c->w_previous = -1.;
   const long long xs = (long long)N * nrhs;
-  Shape sh{nmax, Ragged{c->d_roff.as<long long>(), c->d_rord.as<int>(), ord.data(), off.data()}};
+  Shape sh{nmax, Ragged{c->d_roff.as<long long>(), c->d_rord.as<int>(), ord.data(), off.data()}, wide};
   if (c->mode == NEMOH_B200_FP64) sh.images = fp64_images(c, nsys, sh, headroom);
   OmegaParams* hom = c->h_oms.as<OmegaParams>();
   auto host_setup = [&](int j) {
@@ -1007,6 +1022,7 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
   for (const AsmGroup& g : groups)
     sig.insert(sig.end(), {g.ninfd, g.nfd, g.n_infd, g.n_fd, (long long)g.slot_rk_infd, (long long)g.slot_rk_fd});
   sig.insert(sig.end(), ord.begin(), ord.end());
+  sig.insert(sig.end(), sh.wide.begin(), sh.wide.end());
   unsigned long long key = 1469598103934665603ull;   // FNV-1a over the signature
   for (long long v : sig)
     for (int b = 0; b < 8; ++b) key = (key ^ (unsigned long long)((v >> (8 * b)) & 0xff)) * 1099511628211ull;
@@ -1350,7 +1366,8 @@ int nemoh_b200_set_mesh(nemoh_ctx* c, int np, int nfa, int nsymy, const double* 
     c->w_previous = -1.;
     c->nq_state = 0;
     c->rk_valid[0] = c->rk_valid[1] = false;
-    upload_geometry(c, np, nfa, c->nsymy, xyz, m1234, c->d_xyz, c->d_m, c->d_rec, c->d_rows, c->zer, c->gm);
+    upload_geometry(c, np, nfa, c->nsymy, xyz, m1234, c->d_xyz, c->d_m, c->d_rec, c->d_rows, c->zer, c->gm,
+                    c->wide);
   });
 }
 
@@ -1367,7 +1384,8 @@ int nemoh_b200_add_body(nemoh_ctx* c, int np, int nfa, int nsymy, const double* 
     b->g = g;
     b->depth = depth;
     b->nint = nint;
-    upload_geometry(c, np, nfa, b->nsymy, xyz, m1234, b->d_xyz, b->d_m, b->d_rec, b->d_rows, b->zer, b->gm);
+    upload_geometry(c, np, nfa, b->nsymy, xyz, m1234, b->d_xyz, b->d_m, b->d_rec, b->d_rows, b->zer, b->gm,
+                    b->wide);
     const size_t nds_elems = (size_t)nint * nfa * (b->nsymy + 1);
     CK(b->d_nds.ensure(std::max<size_t>(1, nds_elems) * sizeof(double)));
     if (nint) CK(cudaMemcpyAsync(b->d_nds.p, nds, nds_elems * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -2099,6 +2117,48 @@ int nemoh_b200_diag_sweep_timeout(int device, int* status, double* ms) {
     CK(cudaEventElapsedTime(&t, e0.e, e1.e));
     *ms = t;
     CK(cudaMemcpy(status, st.p, sizeof(int), cudaMemcpyDeviceToHost));
+  });
+}
+
+int nemoh_b200_diag_fp64_update(int device, int n, int nsys, const int* orders, int panels, double* a) {
+  if (!a || nsys < 1 || panels < 1 || panels > 2 || n <= panels * LU_OUTER) return NEMOH_B200_EINVAL;
+  for (int s = 0; orders && s < nsys; ++s)
+    if (orders[s] < 1 || orders[s] > (s ? orders[s - 1] : n)) return NEMOH_B200_EINVAL;
+  if (orders && orders[0] != n) return NEMOH_B200_EINVAL;
+  return guarded(nullptr, [&] {
+    CK(cudaSetDevice(device));
+    DevBuf A, off, ord, st;
+    OzWork w;
+    const size_t nn = (size_t)n * n, bytes = nsys * nn * sizeof(double2);
+    CK(A.ensure(bytes));
+    CK(st.ensure(sizeof(int)));
+    CK(w.ensure(nsys, n));
+    CK(cudaMemset(st.p, 0, sizeof(int)));
+    CK(cudaMemcpy(A.p, a, bytes, cudaMemcpyHostToDevice));
+    Ragged rg;
+    if (orders) {
+      std::vector<long long> o(nsys);
+      for (int s = 0; s < nsys; ++s) o[s] = (long long)(s * nn);
+      CK(off.ensure(nsys * sizeof(long long)));
+      CK(ord.ensure(nsys * sizeof(int)));
+      CK(cudaMemcpy(off.p, o.data(), nsys * sizeof(long long), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(ord.p, orders, nsys * sizeof(int), cudaMemcpyHostToDevice));
+      rg.off = off.as<long long>();
+      rg.ord = ord.as<int>();
+    }
+    const Batch b = make_batch<double2>(A.as<double2>(), n, nullptr, nullptr, rg);
+    long long launches = 0;
+    for (int p = 0; p < panels; ++p) {
+      const OzSet cur = oz_set(w, p, 0);
+      oz_prep(cur, oz_stride(w), b, p * LU_OUTER, nsys, 0, launches);
+      oz_apply(cur, p ? oz_set(w, 0, 0) : OzSet(), oz_stride(w), b, p * LU_OUTER, nsys, 0, launches, st.as<int>(),
+               p + 1 < panels);
+    }
+    CK(cudaGetLastError());
+    int status = 0;
+    CK(cudaMemcpy(&status, st.p, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(a, A.p, bytes, cudaMemcpyDeviceToHost));
+    if (status) throw Fail{status, "tensor-core update timed out waiting on its operands"};
   });
 }
 

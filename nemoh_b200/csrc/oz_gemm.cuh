@@ -6,21 +6,33 @@
 // two orders of magnitude wider and exact. So each operand is split into
 // integer slices (the error-free splitting of Ozaki, Ogita, Oishi and Rump):
 // row r of L21 (column c of U12) gets one power-of-two scale 2^e above its
-// largest component over the panel, every component becomes the 55-bit integer
-// V = rint(x 2^(54 - e)), and V its seven balanced base-256 digits
+// largest component over the panel, every component becomes the integer
+// V = rint(x 2^(62 - e)), |V| <= 2^62, and V its eight balanced base-256 digits
 //     V = sum_t d_t 256^t,  d_t in [-128, 127].
-// Slice i holds the digits of weight 256^(6 - i). A product of two slices is
-// exact in INT32 over K = 64 complex (2 * 64 * 7 * 2^14 < 2^31), products of
-// equal i + j share an accumulator (a diagonal), and the diagonals are summed in
-// FP64 with their powers of 256.
+// Slice i holds the digits of weight 256^(7 - i). Products of equal i + j share
+// an INT32 accumulator (a diagonal) over K = 128 complex, exactly (at most 8
+// products of 256 terms of 2^14: 2^25), and the diagonals are summed in FP64 with
+// their powers of 256.
 //
-// Diagonals i + j <= 7 are kept (34 slice products). What is dropped is below
-// 2^-58 of the row's and column's maxima, what the 55-bit rounding loses below
-// 2^-55 of one maximum. Measured on the influence matrices of six hulls (300 to
-// 780 panels, deep and finite depth, 80-bit reference): the factors' and the
-// solutions' errors are those of an FP64 multiply-add chain to within 2%
-// (e.g. 3.5e-16 and 3.6e-16); with the 28 products of i + j <= 6 the solutions'
-// error is up to 45% larger, so the eighth diagonal stays.
+// Diagonals i + j <= 7 are kept (36 slice products; slice 7 only meets slice 0).
+// A component down to 2^-9 of its row's largest is held with all its 53 bits,
+// the rounding of a smaller one is 2^-63 of the scale at most; what is dropped is
+// below 2^-58 of the product of the two scales per k. Both are relative to a row's
+// and a column's largest components, not to the entry that they update, which is
+// far smaller where the panel's columns couple weakly with one another. Measured
+// against 80-bit arithmetic, FP64 multiply-add chain / this form / seven slices
+// of 55 bits (34 products), the 90% and 99.9% quantiles of the factors' errors
+// relative to each entry: cylinder of 528 panels at 1 rad/s 8.8e-16, 2.9e-15 /
+// 7.1e-16, 1.8e-15 / 7.1e-16, 1.9e-15, at 2.5 rad/s 8.6e-16, 8.6e-15 / 7.8e-16,
+// 4.1e-15 / 8.3e-16, 1.4e-14; box of 100 x 20 x 10 m and 608 panels at 2.5 rad/s (90%)
+// 1.4e-15 / 1.3e-15 / 7.1e-15 and its sources (99%) 3.4e-15 / 3.1e-15 / 4.3e-15.
+// The errors relative to the largest entries agree within 6% in all three.
+//
+// How weakly the columns of a panel may couple is bounded by oz_wide: in a mesh
+// whose numbering mixes a small hull with a large one far away the entries that
+// couple them lose digits (1:20 hulls of 334 panels, 200 m apart, taking turns:
+// sources' 99% quantile 2.0e-13 / 6.6e-13 / 7.8e-12; 1:100 and 20 m apart 9.2e-14 /
+// 2.3e-12 / 3.5e-11). Such panels are updated on the FP64 pipe.
 //
 // The complex product is real: A as [Ar | Ai] along k, B as the planes
 // [-Bi; Br; Bi] of 64 columns each, of which Ar multiplies (Br, Bi) and Ai
@@ -30,15 +42,17 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <utility>
+#include <vector>
 
 #include "linalg.cuh"
 #include "tc_gemm.cuh"
 
 namespace nb200 {
 
-constexpr int OZ_S = 7;                          // slices per operand
-constexpr int OZ_D = 8;                          // diagonals kept: i + j <= 7
+constexpr int OZ_S = 8;                          // slices per operand
+constexpr int OZ_BITS = 62;                      // |V| <= 2^62
 constexpr int OZ_M = 128;                        // rows per tile
 constexpr int OZ_N = 64;                         // complex columns per tile (128 accumulator columns: Re, Im)
 constexpr int OZ_KC = 64;                        // complex k per chunk
@@ -56,28 +70,70 @@ constexpr int OZ_THREADS = 128 + 32 * OZ_EPI_WARPS;   // producer, two MMA issue
 constexpr int OZ_EC = OZ_N / (OZ_EPI_WARPS / 4);   // complex columns per epilogue thread
 constexpr int OZ_BATCH = 2;                        // of them loaded at once
 constexpr int OZ_SMEM = OZ_SLOTS * OZ_SLOT + 256 + 2 * 2 * OZ_N * (int)sizeof(double);
-constexpr int OZ_EMIN = -250;                    // smallest scale exponent (rows and columns below it are round-off)
+// Smallest scale exponent: components of rows and columns whose largest is below
+// 2^-250 lose digits below 2^-313. The factors of influence matrices, whose
+// diagonals are O(1), have no such rows but zero ones.
+constexpr int OZ_EMIN = -250;
 // Trailing entries of a batch (summed over its systems that the panel has not
-// finished) from which an update takes this path; below it the FP64 pipe's one launch is as fast as the images and the
-// update, which then cover few SMs. LU in ms, FP64 pipe against this path: 10
-// systems of 420 panels (0.9 M entries) 0.71 / 0.71, 4 of 588 (0.8 M) 0.94 / 0.95,
-// 2 of 894 (1.2 M) 1.08 / 1.08, 4 of 894 (2.3 M) 1.32 / 1.22, 2 of 1,430 (3.4 M)
-// 2.24 / 1.99, 20 of 588 (4.2 M) 1.44 / 1.25, 1 of 2,380 (5.1 M) 4.21 / 3.37, 20 of
-// 2,380 (101 M) 37.0 / 17.2.
+// finished) from which an update takes this path; below it the FP64 pipe's one
+// launch is as fast as the images and the update, which then cover few SMs. LU in
+// ms, FP64 pipe / this path: 10 systems of 420 panels (0.9 M entries) 0.59 / 0.61, 4
+// of 588 (0.8 M) 0.79 / 0.86, 2 of 894 (1.2 M) 1.00 / 1.04, 20 of 420 (1.7 M) 0.69 /
+// 0.66, 4 of 894 (2.3 M) 1.25 / 1.16, 2 of 1,430 (3.4 M) 2.09 / 1.86, 20 of 588
+// (4.2 M) 1.19 / 1.00, 1 of 2,380 (5.1 M) 4.05 / 3.21, 20 of 2,380 (101 M) 37.0 / 16.8.
 constexpr double OZ_MIN_ENTRIES = 1.5e6;
-// Tiles of a full update (summed likewise) from which panel pairs are merged (four per SM): the
-// merged form reads and writes the trailing block once per pair, the corner
-// update it needs is a launch of one tile's latency more. LU in ms, never merged /
-// merged from 148 tiles / from 600: 20 systems of 420 0.77 / 0.81 / 0.78, 10 of 894
-// 1.51 / 1.52 / 1.48, 1 of 2,380 3.41 / 3.40 / 3.37, 20 of 2,380 18.7 / 18.8 / 17.2.
+// Tiles of a full update (summed likewise) from which panel pairs are merged (four
+// per SM): the merged form reads and writes the trailing block once per pair, the
+// corner update it needs is a launch of one tile's latency more. LU in ms, never
+// merged / from 600 tiles / from 148: 20 systems of 420 0.66 / 0.66 / 0.66, 10 of 894
+// 1.46 / 1.44 / 1.41, 1 of 2,380 3.25 / 3.21 / 3.20, 20 of 2,380 18.1 / 16.8 / 16.8.
 constexpr long long OZ_MERGE_TILES = 600;
 
-// The schedule of a tile. Its 68 slice products run in four phases: diagonals 7 ..
+// Panels of the LU (128 consecutive panels of the mesh) whose update stays on the
+// FP64 pipe: those in which the square of the bounding box's diagonal is more than
+// OZ_MAX_SPREAD times the smallest area. A panel of area a couples with one at a
+// distance d by a / (2 pi d^2) at the most, its neighbours with it by 0.1 or so; the
+// digits are relative to the latter. Contiguous parts of one hull stay below:
+// barges, cylinders and spheres of 300 to 4,000 panels and fleets of random hulls
+// of up to 3,000 reach 3.5e4, typically 3e2 to 3e3. Hulls that take turns in the
+// numbering (90% and 99.9% quantiles of the factors' errors per entry at 2.5 rad/s,
+// FP64 chain / slices): equal ones 100 m apart, 4e4: 1.1e-15, 1.6e-14 / 1.1e-15,
+// 2.5e-14; 300 m, 4e5: 1.4e-15, 1.9e-14 / 1.9e-15, 4.1e-13.
+constexpr double OZ_MAX_SPREAD = 4e4;
+inline std::vector<char> oz_wide(int nfa, const double* xyz, const int* m1234) {
+  std::vector<char> wide((nfa + LU_OUTER - 1) / LU_OUTER);
+  for (size_t b = 0; b < wide.size(); ++b) {
+    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, area2 = 1e300, d2 = 0.;
+    for (int i = (int)b * LU_OUTER; i < std::min(nfa, ((int)b + 1) * LU_OUTER); ++i) {
+      const double* v[4];
+      for (int k = 0; k < 4; ++k) {
+        v[k] = xyz + 3 * (size_t)(m1234[4 * i + k] - 1);
+        for (int c = 0; c < 3; ++c) {
+          lo[c] = std::min(lo[c], v[k][c]);
+          hi[c] = std::max(hi[c], v[k][c]);
+        }
+      }
+      double p[3], q[3], a2 = 0.;   // the diagonals, the square of twice the area
+      for (int c = 0; c < 3; ++c) p[c] = v[2][c] - v[0][c], q[c] = v[3][c] - v[1][c];
+      for (int c = 0; c < 3; ++c) {
+        const double x = p[(c + 1) % 3] * q[(c + 2) % 3] - p[(c + 2) % 3] * q[(c + 1) % 3];
+        a2 += x * x;
+      }
+      area2 = std::min(area2, a2);
+    }
+    for (int c = 0; c < 3; ++c) d2 += (hi[c] - lo[c]) * (hi[c] - lo[c]);
+    wide[b] = !(d2 <= OZ_MAX_SPREAD * 0.5 * std::sqrt(area2));
+  }
+  return wide;
+}
+
+// The schedule of a tile. Its 72 slice products run in four phases: diagonals 7 ..
 // 4 of both chunks into the four accumulators, then diagonals 0 .. 3 of both
 // chunks (slices 0 .. 3, loaded again), so that an accumulator is drained once per
 // phase pair and not once per chunk: the FP64 pipe and the tensor pipe do not run
 // at the same time (measured: 384 k cycles of DFMA and 410 k of MMA take 833 k
-// together), and every drained value costs FP64 work.
+// together), and every drained value costs FP64 work. Slice 7 of a chunk, which
+// only meets slice 0, borrows a slot that is free or retires at once.
 // Each step is one slice product (A slice i, B slice j) of a phase. The order lets
 // slices retire early and lets the accumulators finish in pairs, (0, 1) before
 // (2, 3), which are drained and free again before the next phase pair meets them;
@@ -101,15 +157,18 @@ struct OzPhase {
 // slots[i]: slot of slice i (nsl slices); pairs: (i, j) in order; low: diagonals 0
 // .. 3 (accumulator i + j), else 7 .. 4 (accumulator 7 - i - j); begin / end: the
 // first / last chunk of the phase pair. Both issuers wait for and release every
-// slot of the phase (a slot's barrier counts two releases), one that it does not
-// read with its last step.
+// slot of the phase (a slot's barrier counts two releases), one that this issuer
+// does not read with its first step after the other's last read, or with its last.
 template <int N>
 constexpr OzPhase<N> oz_phase(const int (&pairs)[N][2], const int (&slots)[OZ_S], int nsl, bool low, bool begin,
                               bool end, int mine) {
   OzPhase<N> p{};
   int all = 0;
   for (int i = 0; i < nsl; ++i) all |= 1 << slots[i];
-  int seen = 0, used = 0;
+  int seen = 0, used = 0, reads = 0;
+  for (int k = 0; k < N; ++k)
+    if ((mine >> (low ? pairs[k][0] + pairs[k][1] : 7 - pairs[k][0] - pairs[k][1])) & 1)
+      reads |= (1 << slots[pairs[k][0]]) | (1 << slots[pairs[k][1]]);
   for (int k = 0; k < N; ++k) {
     const int i = pairs[k][0], j = pairs[k][1], acc = low ? i + j : 7 - i - j;
     if (!((mine >> acc) & 1)) continue;
@@ -129,7 +188,9 @@ constexpr OzPhase<N> oz_phase(const int (&pairs)[N][2], const int (&slots)[OZ_S]
       later |= (1 << slots[pairs[q][0]]) | (1 << slots[pairs[q][1]]);
       open |= 1 << a;
     }
-    if (later == 0) m |= all & ~(seen | m);   // the last step
+    int ahead = 0;   // slots that either issuer reads from here on
+    for (int q = k; q < N; ++q) ahead |= (1 << slots[pairs[q][0]]) | (1 << slots[pairs[q][1]]);
+    m |= (later == 0 ? all : all & ~(reads | ahead)) & ~seen;
     t.need = (short)(m & ~seen);
     seen |= m;
     t.retire = (short)(m & ~later);
@@ -137,16 +198,16 @@ constexpr OzPhase<N> oz_phase(const int (&pairs)[N][2], const int (&slots)[OZ_S]
   }
   return p;
 }
-constexpr int OZ_P0[24][2] = {{1, 6}, {6, 1}, {1, 5}, {5, 1}, {1, 4}, {4, 1}, {0, 6}, {6, 0},
-                              {0, 5}, {5, 0}, {0, 4}, {4, 0}, {2, 5}, {5, 2}, {2, 4}, {4, 2},
+constexpr int OZ_P0[26][2] = {{1, 6}, {6, 1}, {1, 5}, {5, 1}, {1, 4}, {4, 1}, {0, 7}, {7, 0}, {0, 6},
+                              {6, 0}, {0, 5}, {5, 0}, {0, 4}, {4, 0}, {2, 5}, {5, 2}, {2, 4}, {4, 2},
                               {2, 2}, {3, 4}, {4, 3}, {3, 3}, {2, 3}, {3, 2}, {1, 3}, {3, 1}};
-constexpr int OZ_P1[24][2] = {{1, 6}, {6, 1}, {1, 5}, {5, 1}, {0, 6}, {6, 0}, {2, 5}, {5, 2},
-                              {2, 4}, {4, 2}, {3, 4}, {4, 3}, {3, 3}, {0, 5}, {5, 0}, {1, 4},
+constexpr int OZ_P1[26][2] = {{1, 6}, {6, 1}, {1, 5}, {5, 1}, {0, 6}, {6, 0}, {2, 5}, {5, 2}, {2, 4},
+                              {4, 2}, {0, 7}, {7, 0}, {3, 4}, {4, 3}, {3, 3}, {0, 5}, {5, 0}, {1, 4},
                               {4, 1}, {2, 3}, {3, 2}, {0, 4}, {4, 0}, {1, 3}, {3, 1}, {2, 2}};
 constexpr int OZ_P2[10][2] = {{0, 0}, {0, 1}, {1, 0}, {1, 1}, {0, 2}, {2, 0}, {1, 2}, {2, 1}, {0, 3}, {3, 0}};
 constexpr int OZ_P3[10][2] = {{0, 0}, {0, 1}, {1, 0}, {0, 2}, {2, 0}, {1, 1}, {1, 2}, {2, 1}, {0, 3}, {3, 0}};
-constexpr int OZ_L0[OZ_S] = {0, 1, 2, 3, 4, 5, 6}, OZ_L1[OZ_S] = {0, 7, 2, 3, 4, 5, 6},
-              OZ_L2[OZ_S] = {6, 1, 5, 4, 0, 0, 0}, OZ_L3[OZ_S] = {0, 7, 2, 3, 0, 0, 0};
+constexpr int OZ_L0[OZ_S] = {0, 1, 2, 3, 4, 5, 6, 7}, OZ_L1[OZ_S] = {0, 7, 2, 3, 4, 5, 6, 1},
+              OZ_L2[OZ_S] = {6, 1, 5, 4}, OZ_L3[OZ_S] = {0, 7, 2, 3};
 // Two warps issue, each with two of the accumulators: an MMA is handed over only
 // about when the one before it starts (measured: a pause of 200 cycles after every
 // four MMAs costs 219), so one issuer's waits and releases would leave the tensor
@@ -154,17 +215,17 @@ constexpr int OZ_L0[OZ_S] = {0, 1, 2, 3, 4, 5, 6}, OZ_L1[OZ_S] = {0, 7, 2, 3, 4,
 constexpr int OZ_WHO0 = (1 << 0) | (1 << 3), OZ_WHO1 = (1 << 1) | (1 << 2);
 template <int WHO>
 struct OzPlan {
-  static constexpr OzPhase<24> p0 = oz_phase(OZ_P0, OZ_L0, 7, false, true, false, WHO);
-  static constexpr OzPhase<24> p1 = oz_phase(OZ_P1, OZ_L1, 7, false, false, true, WHO);
+  static constexpr OzPhase<26> p0 = oz_phase(OZ_P0, OZ_L0, 8, false, true, false, WHO);
+  static constexpr OzPhase<26> p1 = oz_phase(OZ_P1, OZ_L1, 8, false, false, true, WHO);
   static constexpr OzPhase<10> p2 = oz_phase(OZ_P2, OZ_L2, 4, true, true, false, WHO);
   static constexpr OzPhase<10> p3 = oz_phase(OZ_P3, OZ_L3, 4, true, false, true, WHO);
 };
-// the loads of a tile in the order their slots free up: nibbles slice, slot
-constexpr int OZ_LOADS = 22;
+// the loads of a tile in the order their slots free up
+constexpr int OZ_LOADS = 24;
 constexpr signed char OZ_LOAD[OZ_LOADS][3] = {   // slice, slot, chunk
-    {1, 1, 0}, {6, 6, 0}, {5, 5, 0}, {4, 4, 0}, {0, 0, 0}, {2, 2, 0}, {3, 3, 0},
-    {1, 7, 1}, {6, 6, 1}, {0, 0, 1}, {5, 5, 1}, {4, 4, 1}, {2, 2, 1}, {3, 3, 1},
-    {1, 1, 0}, {0, 6, 0}, {2, 5, 0}, {3, 4, 0},
+    {1, 1, 0}, {6, 6, 0}, {5, 5, 0}, {4, 4, 0}, {7, 7, 0}, {0, 0, 0}, {2, 2, 0}, {3, 3, 0},
+    {1, 7, 1}, {6, 6, 1}, {0, 0, 1}, {5, 5, 1}, {4, 4, 1}, {2, 2, 1}, {7, 1, 1}, {3, 3, 1},
+    {0, 6, 0}, {1, 1, 0}, {2, 5, 0}, {3, 4, 0},
     {0, 0, 1}, {1, 7, 1}, {2, 2, 1}, {3, 3, 1}};
 
 // Operand images and scales of two panels (the update of one panel may be
@@ -231,8 +292,8 @@ inline OzSet oz_set(const OzWork& w, int set, int s0) {
   return r;
 }
 
-// 16 components scaled by 2^(54 - e): their digits, slice by slice, as 16-byte
-// rows out(i, uint4). V + 0x0080..80 has the digits offset by 128 as its bytes,
+// 16 components scaled by 2^(62 - e): their digits, slice by slice, as 16-byte
+// rows out(i, uint4). V + 0x8080..80 has the digits offset by 128 as its bytes,
 // so the digits are those bytes with the top bit flipped.
 template <class Out>
 __device__ __forceinline__ void oz_digits(const double* x, double scale, bool neg, Out out) {
@@ -245,11 +306,11 @@ __device__ __forceinline__ void oz_digits(const double* x, double scale, bool ne
       long long v = __double2ll_rn(x[4 * q + j] * scale);
       if (neg) v = -v;
       const unsigned long long u =
-          ((unsigned long long)(v + 0x0080808080808080ll)) ^ 0x0080808080808080ull;
+          ((unsigned long long)v + 0x8080808080808080ull) ^ 0x8080808080808080ull;
       lo[j] = (uint32_t)u;
       hi[j] = (uint32_t)(u >> 32);
     }
-    // byte t of the four values, in order, is the word of slice 6 - t
+    // byte t of the four values, in order, is the word of slice 7 - t
     auto quad = [](const uint32_t* v, uint32_t& b0, uint32_t& b1, uint32_t& b2, uint32_t& b3) {
       const uint32_t p = __byte_perm(v[0], v[1], 0x5140), q2 = __byte_perm(v[2], v[3], 0x5140);
       const uint32_t r = __byte_perm(v[0], v[1], 0x7362), s = __byte_perm(v[2], v[3], 0x7362);
@@ -258,9 +319,8 @@ __device__ __forceinline__ void oz_digits(const double* x, double scale, bool ne
       b2 = __byte_perm(r, s, 0x5410);
       b3 = __byte_perm(r, s, 0x7632);
     };
-    uint32_t top;
-    quad(lo, w[6][q], w[5][q], w[4][q], w[3][q]);
-    quad(hi, w[2][q], w[1][q], w[0][q], top);
+    quad(lo, w[7][q], w[6][q], w[5][q], w[4][q]);
+    quad(hi, w[3][q], w[2][q], w[1][q], w[0][q]);
   }
 #pragma unroll
   for (int i = 0; i < OZ_S; ++i) out(i, make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]));
@@ -274,7 +334,7 @@ __device__ __forceinline__ unsigned oz_mag(double x, unsigned m) {
 __device__ __forceinline__ int oz_exponent(unsigned mag) { return max((int)(mag >> 20) - 1022, OZ_EMIN); }
 __device__ __forceinline__ double oz_pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 // what one row's digits are worth in the result: the kept diagonals weigh
-// 256^7 .. 1 in units of 256^5 of both operands, 2^20 of each. A row with a
+// 256^7 .. 1 in units of 256^7, 2^28 of each operand. A row with a
 // NaN or an infinity makes every result of the row NaN.
 __device__ __forceinline__ double oz_scale(unsigned mag, int e) {
   return mag >= 0x7ff00000u ? __longlong_as_double(0x7ff8000000000000ll) : oz_pow2(e - 34);
@@ -283,7 +343,7 @@ __device__ __forceinline__ double oz_scale(unsigned mag, int e) {
 // Images of the panel [k0, k0 + 128): L21 = A[r1:n, k0:r1] and U12 = A[k0:r1,
 // r1:n], r1 = k0 + 128. Blocks [0, na): 32 rows of L21, thread = (row, 16 k);
 // the others: 32 columns of U12, thread = (column, 16 k). Reads 16 B and writes
-// 14 B (L21) or 21 B (U12) per entry, bound by HBM and the FP64 -> INT64
+// 16 B (L21) or 24 B (U12) per entry (two systems of 2,252 rows: 14.5 us), bound by HBM and the FP64 -> INT64
 // conversions; one pass over the operands, which stay in registers between the
 // maximum and the digits.
 constexpr int OZP_THREADS = 256;
@@ -322,7 +382,7 @@ __global__ void __launch_bounds__(OZP_THREADS) oz_prep_kernel(Batch b, int k0, O
     for (int o = 4; o > 0; o >>= 1) mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, o));
   }
   const int e = oz_exponent(mag);
-  const double sc = oz_pow2(54 - e);
+  const double sc = oz_pow2(OZ_BITS - e);
   const int ch = g / (OZ_KC / 16), kg = g % (OZ_KC / 16);
   if (isA) {
     if (g == 0) s.ra[blockIdx.z * st.s + rr] = oz_scale(mag, e);
@@ -534,10 +594,11 @@ __device__ __forceinline__ void oz_subtract(double2* C, int n, int ncol, double 
 // What bounds it: the tensor pipe at 64 cycles an MMA (an N = 128 MMA reads its
 // operands from shared memory at the port's 128 B a cycle), the FP64 and integer
 // work of the drains, which takes tensor cycles, and the read-modify-write of A22,
-// 256 KB per tile. Two systems of 2,252 trailing rows: 193 us per panel (1,296
-// tiles, 17,400 cycles of MMAs each; 113 us without drains and A22), 286 us for a
-// merged pair; a first form that drained every 64 complex k took 256 and 420 us,
-// the FP64 pipe 830 us per panel.
+// 256 KB per tile. Two systems of 2,252 trailing rows: 205 us per panel (1,296
+// tiles, 18,400 cycles of MMAs each), 299 us for a merged pair, 27 us for a corner.
+// With seven slices per operand (17,400 cycles) 198, 291 and 25 us, of which 113
+// without drains and A22; a first form that drained every 64 complex k took 256 and
+// 420 us, the FP64 pipe 830 us per panel.
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     oz_update_kernel(Batch b, int k0, OzSet cur, OzSet prev, OzStride st, int nsys, int* status, int nti, int ntc,
                      int corner) {
