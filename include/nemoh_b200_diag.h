@@ -34,6 +34,10 @@ int nemoh_b200_diag_fp64_peak(int device, double* tflops);
  * graph do not count) */
 struct nemoh_ctx;
 long long nemoh_b200_diag_tensor_updates(const struct nemoh_ctx* ctx);
+/* the kernels' short reciprocals of n values each: rs = 1 / sqrt(x) of the wave
+ * pass, rp = 1 / p of the FP64 and rq = 1 / q of the FP32 pivots (complex) */
+int nemoh_b200_diag_reciprocals(int device, int n, const double* x, double* rs, const double* p, double* rp,
+                                const float* q, float* rq);
 /* the tensor-core trailing update by itself, on host matrices: `nsys` complex
  * column-major matrices n * n elements apart, of order n (orders null) or
  * orders[s] <= n, decreasing, orders[0] = n (leading dimension orders[s]).

@@ -1978,6 +1978,15 @@ int nemoh_b200_last_factor_ms(nemoh_ctx* c, double* lu_ms) {
 // ---------------------------------------------------------------------------
 #include "../../include/nemoh_b200_diag.h"
 
+// the short reciprocals in place: rsqrt3 of x, crecip of p and q
+static __global__ void reciprocals_kernel(int n, double* x, double2* p, float2* q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  x[i] = rsqrt3(x[i]);
+  p[i] = crecip(p[i]);
+  q[i] = crecip(q[i]);
+}
+
 extern "C" {
 
 int nemoh_b200_diag_dispersion_root(double ak, double* root) { return finite_depth_root(ak, root); }
@@ -2117,6 +2126,26 @@ int nemoh_b200_diag_sweep_timeout(int device, int* status, double* ms) {
     CK(cudaEventElapsedTime(&t, e0.e, e1.e));
     *ms = t;
     CK(cudaMemcpy(status, st.p, sizeof(int), cudaMemcpyDeviceToHost));
+  });
+}
+
+int nemoh_b200_diag_reciprocals(int device, int n, const double* x, double* rs, const double* p, double* rp,
+                                const float* q, float* rq) {
+  if (n < 1 || !x || !rs || !p || !rp || !q || !rq) return NEMOH_B200_EINVAL;
+  return guarded(nullptr, [&] {
+    CK(cudaSetDevice(device));
+    DevBuf dx, dp, dq;
+    CK(dx.ensure((size_t)n * sizeof(double)));
+    CK(dp.ensure((size_t)n * sizeof(double2)));
+    CK(dq.ensure((size_t)n * sizeof(float2)));
+    CK(cudaMemcpy(dx.p, x, (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dp.p, p, (size_t)n * sizeof(double2), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dq.p, q, (size_t)n * sizeof(float2), cudaMemcpyHostToDevice));
+    reciprocals_kernel<<<(n + 255) / 256, 256>>>(n, dx.as<double>(), dp.as<double2>(), dq.as<float2>());
+    CK(cudaGetLastError());
+    CK(cudaMemcpy(rs, dx.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(rp, dp.p, (size_t)n * sizeof(double2), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(rq, dq.p, (size_t)n * sizeof(float2), cudaMemcpyDeviceToHost));
   });
 }
 

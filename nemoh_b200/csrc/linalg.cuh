@@ -108,9 +108,11 @@ __device__ __forceinline__ double cabs2(float2 a) { return hypotf(a.x, a.y); }
 
 // reciprocal of a pivot, scaled by a power of two so that |p|^2 neither
 // overflows nor underflows. Every elimination step waits for it, so 1 / d with
-// d in [1, 8) is the hardware's approximation and one Householder step (third
-// order in double precision: 2^-20 to below 2^-58; second order in single),
-// without the special cases of a general quotient.
+// d in [1, 8) is the hardware's approximation and one step of Householder's
+// method, r (1 + h + h^2) with h = 1 - d r (cubic convergence, 2^-20 to 2^-57) in
+// double, Newton's r (1 + h) in single precision, without the special cases of a
+// general quotient. Each component's error is below 4.1 roundings (two of d, one of
+// the step, one of the product); the tests hold both forms to that.
 __device__ __forceinline__ double2 crecip(double2 p) {
   const int e = max(__double2hiint(p.x) & 0x7ff00000, __double2hiint(p.y) & 0x7ff00000) >> 20;
   const double s = __hiloint2double(max(1, 2046 - e) << 20, 0);
