@@ -276,12 +276,10 @@ __global__ void __launch_bounds__(ASM_ROWS, ASM_MINB_RANKINE) rankine_cache_kern
 
 // ---------------------------------------------------------------------------
 // Wave pass over the upper triangle of 16 x 16 tiles: a pair of submerged
-// panels is evaluated once for both orders (finite depth: wave_fd_sym and the
-// exponential images of the same branch, fd_images_pair; deep water:
-// wave_infd_both), any other pair once per order (pair_wave); both the tile
-// and its transpose are added to the real parts and written to the imaginary
-// parts, the tile straight from the evaluating threads, its transpose column
-// by column through shared memory.
+// panels is evaluated once for both orders (wave_sym_pair), any other pair once
+// per order (pair_wave_ordered); both the tile and its transpose are added to the
+// real parts and written to the imaginary parts, the tile straight from the
+// evaluating threads, its transpose column by column through shared memory.
 // ---------------------------------------------------------------------------
 constexpr int WS_T = 16;
 constexpr int WS_THREADS = 128;
@@ -364,6 +362,22 @@ NB_HD __forceinline__ void wave_infd_both(const GreenCtx& g, const OmegaParams& 
     }
   }
   wave_combine<false>(om, PI.aire, NJJ, w, PJ.xn, PJ.yn, PJ.zn, oji);
+}
+
+// both orders of a pair of submerged panels; false where the reference's wave term
+// is undefined (AKZ > -1.5E-6). Finite depth: the exponential images first, while
+// nothing of the tabulated part is live (their loop keeps to the registers), then
+// the tabulated part of the same branch on top of them.
+template <bool FD>
+NB_HD __forceinline__ bool wave_sym_pair(const GreenCtx& g, const OmegaParams& om, const PanelRec& PI,
+                                              const PanelRec& PJ, int NJJ, bool both, PairOut& oij, PairOut& oji) {
+  if (FD) {
+    oij = oji = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
+    fd_images_pair(g, om, PI, PJ, NJJ, both, oij, oji);
+    return wave_fd_sym_add(g, om, PI, PJ, NJJ, both, oij, oji);
+  }
+  wave_infd_both(g, om, PI, PJ, NJJ, both, oij, oji);
+  return true;
 }
 
 // Transposed results of a tile, one array per PairOut field, rows padded to
@@ -460,15 +474,7 @@ __global__ void __launch_bounds__(WS_THREADS, FD ? ASM_MINB_WAVE_FD : ASM_MINB_W
     PairOut oij, oji;
     if (!lv) {
     } else if (PI.zg < g.zer && PJ.zg < g.zer) {
-      if (FD) {
-        // the images first, while nothing of the tabulated part is live: their
-        // loop keeps to the registers
-        oij = oji = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
-        fd_images_pair(g, som, PI, PJ, NJJ, both, oij, oji);
-        if (!wave_fd_sym_add(g, som, PI, PJ, NJJ, both, oij, oji)) set_status(g.status, ST_AKZ_UNDEFINED);
-      } else {
-        wave_infd_both(g, som, PI, PJ, NJJ, both, oij, oji);
-      }
+      if (!wave_sym_pair<FD>(g, som, PI, PJ, NJJ, both, oij, oji)) set_status(g.status, ST_AKZ_UNDEFINED);
     } else {
       pair_wave_ordered<FD>(g, som, PI, PJ, oij);
       if (both) pair_wave_ordered<FD>(g, som, PJ, PI, oji);

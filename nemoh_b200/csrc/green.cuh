@@ -770,6 +770,7 @@ NB_HD __forceinline__ bool wave_fd_sym_add(const GreenCtx& g, const OmegaParams&
   return true;
 }
 
+// the tabulated part alone, as host checks of it take it
 NB_HD __forceinline__ bool wave_fd_sym(const GreenCtx& g, const OmegaParams& om, const PanelRec& PI,
                                             const PanelRec& PJ, int NJJ, bool both, PairOut& oij, PairOut& oji) {
   const PairOut zero = PairOut{0, 0, 0, 0, 0, 0, 0, 0};
