@@ -563,6 +563,13 @@ bool fp64_images(nemoh_ctx* c, int nsys, const Shape& sh, bool headroom = false)
   bool any = false;
   for (int k0 = 0; k0 + LU_OUTER < sh.n; k0 += LU_OUTER) any |= !sh.wide_panel(k0);
   if (!any) return false;
+  if (c->oz.grows(nsys, sh.n)) {   // images that can't grow stay for the batches that they are large enough for
+    size_t fr = 0, tot = 0;
+    CK(cudaMemGetInfo(&fr, &tot));
+    const size_t need = nsys * oz_bytes_per_system(sh.n), room = fr + c->oz.bytes();
+    if (need > room) return false;
+    headroom = headroom && need + need / 4 <= room;
+  }
   return c->oz.ensure(nsys, sh.n, headroom) == cudaSuccess;
 }
 
@@ -855,6 +862,12 @@ void solve_frequencies_impl(nemoh_ctx* c, int nomega, const double* omegas, int 
 // system of the batch.
 // ---------------------------------------------------------------------------
 
+// device bytes of the operand images of one item's FP64 updates, in a ragged batch
+// whose largest order is nmax
+size_t item_image_bytes(const nemoh_ctx* c, const BodyState& b, int nmax) {
+  return c->mode == NEMOH_B200_FP64 && nmax > LU_OUTER ? (b.nsymy + 1) * oz_bytes_per_system(nmax) : 0;
+}
+
 // device bytes one item adds to a ragged batch whose largest order is nmax
 size_t item_bytes(const nemoh_ctx* c, const BodyState& b, int nmax, int nrhs) {
   const size_t n = b.nfa, cls = b.nsymy + 1, nm = nmax, nblk = (nm + TB - 1) / TB;
@@ -865,10 +878,9 @@ size_t item_bytes(const nemoh_ctx* c, const BodyState& b, int nmax, int nrhs) {
     mats += n * n * sizeof(float2);
     per_sys += nm * nrhs * (2 * sizeof(double2) + 2 * sizeof(float2)) + (DIAG_SCRATCH + PINV_SCRATCH) * sizeof(float2) +
                nblk * 2 * TB * TB * sizeof(float2) + tc_bytes_per_system(nm);
-  } else if (nm > LU_OUTER) {
-    per_sys += oz_bytes_per_system(nm);
   }
-  return cls * (mats + per_sys) + sizeof(OmegaParams) + sizeof(SlotMesh) + sizeof(ItemDesc);
+  return cls * (mats + per_sys) + item_image_bytes(c, b, nmax) + sizeof(OmegaParams) + sizeof(SlotMesh) +
+         sizeof(ItemDesc);
 }
 
 // one ragged batch: items[0..k) index the caller's arrays, already in
@@ -1159,13 +1171,16 @@ void solve_bodies_impl(nemoh_ctx* c, int nitem, const int* body, const double* o
   CK(cudaEventRecord(rk1.e, c->stream));
   // admission by HBM footprint: 80% of the free memory, the batch's own
   // buffers counted as free
+  auto held_bytes = [&] {   // but for the images
+    return c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes + c->d_diag.bytes +
+           c->mixed.bytes();
+  };
   auto free_bytes = [&] {
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
     // the FP64 updates' images are a mixed batch's only while it falls back
     const size_t images = c->mode == NEMOH_B200_FP64 ? c->oz.bytes() : 0;
-    return (size_t)((fr + c->d_D.bytes + c->d_S.bytes + c->d_X.bytes + c->d_Y.bytes + c->d_inv.bytes +
-                     c->d_diag.bytes + c->mixed.bytes() + images) * 0.8);
+    return (size_t)((fr + held_bytes() + images) * 0.8);
   };
   size_t budget = free_bytes();
   if (c->mode == NEMOH_B200_MIXED && c->oz.bytes()) {   // an earlier fallback's: given back where the call needs the room
@@ -1185,14 +1200,29 @@ void solve_bodies_impl(nemoh_ctx* c, int nitem, const int* body, const double* o
   int pos = 0;
   while (pos < nitem) {
     const int nmax = c->bodies[body[idx[pos]]]->nfa;
-    size_t used = 0;
+    size_t used = 0, images = 0;
     int end = pos;
     while (end < nitem) {
-      const size_t need = item_bytes(c, *c->bodies[body[idx[end]]], nmax, nrhs);
+      const BodyState& b = *c->bodies[body[idx[end]]];
+      const size_t need = item_bytes(c, b, nmax, nrhs);
       if (end > pos && used + need > budget) break;
       used += need;
+      images += item_image_bytes(c, b, nmax);
       ++end;
     }
+    // The matrices of smaller hulls are a smaller part of their batch and its images
+    // a larger one, while the buffers keep the size that the batches of larger hulls
+    // gave them: the images may fill the budget and an eighth (0.9 of the free
+    // memory) beside what is held, and the batch is cut to that. Where less than a
+    // quarter of them fits, its updates run on the FP64 pipe instead.
+    const size_t others = std::max(held_bytes(), used - images), most = budget + budget / 8;
+    const size_t room = std::max(c->oz.bytes(), most > others ? most - others : 0);
+    if (images > room && images / 4 <= room)
+      for (; end > pos + 1 && images > room; --end) {
+        const BodyState& b = *c->bodies[body[idx[end - 1]]];
+        used -= item_bytes(c, b, nmax, nrhs);
+        images -= item_image_bytes(c, b, nmax);
+      }
     // the buffers' growth headroom (a quarter) only where the batch leaves room
     ragged_batch(c, idx.data() + pos, end - pos, body, omegas, nrhs, nvel_off, force_off, nvel_d, force_d,
                  used + used / 4 <= budget);

@@ -249,6 +249,11 @@ struct OzWork {
     have_a = have_b = have_sc = 0;
   }
   ~OzWork() { release(); }
+  bool grows(int ns, int n) const {
+    const size_t t = 2 * (size_t)ns * ((n + OZ_M - 1) / OZ_M);
+    return t * OZ_NCH * OZ_S * OZ_A > have_a || t * 2 * OZ_NCH * OZ_S * OZ_B > have_b ||
+           t * 2 * OZ_M * sizeof(double) > have_sc;
+  }
   // all of the images or none of them
   cudaError_t ensure(int ns, int n, bool headroom = false) {
     tiles = (n + OZ_M - 1) / OZ_M;

@@ -179,3 +179,45 @@ def test_small_systems_are_not_charged_for_images(monkeypatch):
         whole = launches(s)
         monkeypatch.setenv("NEMOH_B200_BATCH_BYTES", str(64 * MB))
         assert launches(s) == whole
+
+
+def test_batches_of_one_call_share_the_room_for_images(monkeypatch):
+    """A call of two batches, the small hulls' second: their matrices are smaller and
+    their images larger than those of the first, and the buffers keep their size, so that
+    images for a whole budget of small hulls don't fit beside them. The batch is cut to
+    the room, both take the tensor cores, and every call finds the buffers where the last
+    one left them: its batches replay."""
+    monkeypatch.setenv("NEMOH_B200_BATCH_BYTES", str(400 * MB))
+    rng = np.random.default_rng(6)
+    om_a, nv_a = _items(rng, 1400, 5)     # 62 MB of matrices and 14 MB of images each
+    om_b, nv_b = _items(rng, 400, 36)     # 5 MB and 5 MB
+    body = np.array([0] * 5 + [1] * 36, np.int32)
+    om, nv = np.concatenate([om_a, om_b]), nv_a + nv_b
+
+    def bodies(s):
+        s.add_body(_body(1400))
+        s.add_body(_body(400))
+        s.prepare_bodies()
+
+    with nb.Solver(0, nb.FP64) as s:
+        bodies(s)
+        ref = [s.solve_bodies(body[:5], om[:5], nv[:5]), s.solve_bodies(body[5:], om[5:], nv[5:])]
+        ref = ref[0] + ref[1]
+        large = s.tensor_updates()
+        s.solve_bodies(body[:5], om[:5], nv[:5])
+        large = s.tensor_updates() - large
+    with nb.Solver(0, nb.FP64) as s:
+        bodies(s)
+        s.solve_bodies(body[6:7], om[6:7], nv[6:7])   # kernels loaded
+        before = s.tensor_updates()
+        with _only(490 * MB):
+            runs = [s.solve_bodies(body, om, nv)]     # the buffers grow from batch to batch
+            assert s.tensor_updates() - before > large > 0
+            s.set_graphs(True)   # one call directly, one captured, two replayed
+            runs += [s.solve_bodies(body, om, nv) for _ in range(4)]
+        captures, replays = s.graph_stats()
+        assert captures >= 2 and replays == 2 * captures
+    for got in runs:
+        for g, r in zip(got, ref):
+            # both are backward-stable solves of well-conditioned systems
+            assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
