@@ -1029,8 +1029,11 @@ void ragged_batch(nemoh_ctx* c, const int* items, int k, const int* body, const 
                                 (long long)c->mixed.inv, (long long)c->mixed.pinv, (long long)c->mixed.norms,
                                 (long long)c->mixed.state, (long long)c->mixed.tc.a, (long long)c->mixed.tc.b,
                                 (long long)c->mixed.tc.wv, (long long)c->mixed.flow, (long long)c->mixed.act,
-                                (long long)c->d_flow.p, (long long)c->oz.a, (long long)c->oz.b, (long long)c->oz.sc,
-                                (long long)sh.images};
+                                (long long)c->d_flow.p, (long long)sh.images,
+                                // the images only where the sequence holds them: a mixed batch's
+                                // FP64 fallback runs outside it, with images of its own size
+                                sh.images ? (long long)c->oz.a : 0, sh.images ? (long long)c->oz.b : 0,
+                                sh.images ? (long long)c->oz.sc : 0};
   for (const AsmGroup& g : groups)
     sig.insert(sig.end(), {g.ninfd, g.nfd, g.n_infd, g.n_fd, (long long)g.slot_rk_infd, (long long)g.slot_rk_fd});
   sig.insert(sig.end(), ord.begin(), ord.end());

@@ -221,3 +221,29 @@ def test_batches_of_one_call_share_the_room_for_images(monkeypatch):
         for g, r in zip(got, ref):
             # both are backward-stable solves of well-conditioned systems
             assert np.abs(g - r).max() <= 1e-11 * np.abs(r).max()
+
+
+def test_mixed_batches_that_fall_back_replay(monkeypatch):
+    """The FP64 fallback of a mixed batch runs outside the captured sequence: its
+    images, which another batch's fallback has moved, are no reason to capture anew."""
+    rng = np.random.default_rng(7)
+    om_a, nv_a = _items(rng, 1000, 20)   # images of 210 MB
+    om_b, nv_b = _items(rng, 300, 60)    # of 236 MB; of the other buffers the fallback's are smaller
+    with nb.Solver(0, nb.MIXED) as s:
+        s.add_body(_body(1000))
+        s.add_body(_body(300))
+        s.prepare_bodies()
+        s.solve_bodies(np.ones(60, np.int32), om_b, nv_b)
+        assert s.fallback_count()[0] == 0
+        monkeypatch.setenv("NEMOH_B200_REFINE_MAX_IT", "1")   # every system falls back
+        s.solve_bodies(np.zeros(20, np.int32), om_a, nv_a)
+        s.set_graphs(True)
+        for _ in range(2):
+            s.solve_bodies(np.zeros(20, np.int32), om_a, nv_a)
+        assert s.graph_stats() == (1, 0)
+        updates = s.tensor_updates()
+        s.solve_bodies(np.ones(60, np.int32), om_b, nv_b)
+        assert s.tensor_updates() > updates
+        s.solve_bodies(np.zeros(20, np.int32), om_a, nv_a)
+        assert s.fallback_count()[0] == 5
+        assert s.graph_stats() == (1, 1)
