@@ -1186,7 +1186,9 @@ void solve_bodies_impl(nemoh_ctx* c, int nitem, const int* body, const double* o
     return (size_t)((fr + held_bytes() + images) * 0.8);
   };
   size_t budget = free_bytes();
-  if (c->mode == NEMOH_B200_MIXED && c->oz.bytes()) {   // an earlier fallback's: given back where the call needs the room
+  // an earlier fallback's images are given back where the call needs the room and they
+  // are more than a trifle of it (those of one or two systems stay)
+  if (c->mode == NEMOH_B200_MIXED && c->oz.bytes() > budget / 64) {
     size_t need = 0;
     for (int i : idx) need += item_bytes(c, *c->bodies[body[i]], c->bodies[body[idx[0]]]->nfa, nrhs);
     if (need > budget) {
