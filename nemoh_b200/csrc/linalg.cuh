@@ -10,11 +10,12 @@
 //   lu_diag_kernel    factor A11 once per system, invert L11 and U11
 //   lu_panel_kernel   L21 <- A21 U11^-1, U12 <- L11^-1 A12, store factored A11
 //   zgemm_update      A22 <- A22 - L21 U12 over any rectangle of A22
-// Small FP64 systems update the whole trailing matrix after every step; large FP64
-// batches (oz_gemm.cuh) defer it outside a 128-column panel to exact INT8 slice
-// products on the tensor cores, and the mixed
-// path (mixed.cuh) to one split-BF16
-// tensor-core product per panel.
+// Both paths work in two levels: inside a 128-column panel the steps above, the
+// rest of the trailing matrix once per panel (lu_two_level) - in FP64 by
+// zgemm_update or, in batches of enough trailing entries, by exact INT8 slice
+// products on the tensor cores (oz_gemm.cuh), in the mixed path (mixed.cuh) by
+// split-BF16 products on them. Only the allocation-free entry point, which has no
+// room for a panel's scratch, updates the whole trailing matrix after every step.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(128) zgemm_update_kernel(BatchT<C2> b, int k, 
 // The same update by 32 x 32 tiles, inner dimension in chunks of 32 held whole in
 // shared memory: thread = one row, four columns. A 64 x 64 tile keeps its one
 // warp per scheduler waiting on its chunks and takes 39 us at least for K = 128;
-// this form gives four times the CTAs, six to an SM. FP64, K = 128, us against
+// this form gives four times the CTAs, two to an SM (120 registers). FP64, K = 128, us against
 // the 64 x 64 tiles: 12 / 39 for one system of 300, 59 / 63 for four of 600, 351
 // / 351 for ten of 900 (5,760 tiles), 867 / 799 for ten of 1,400; K = 32, twenty
 // systems of 1,200: 35 / 64 inside the panel, 33 / 52 for its row strip.

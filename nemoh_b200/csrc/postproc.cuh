@@ -5,8 +5,9 @@
 // with t_i = i dt. Coefficients are (Nw, Nrad, Nint) with w fastest, K is
 // (Ntime, Nrad, Nint) with time fastest. A thread of K owns one time and up to
 // IRF_CH radiation/force pairs; a CTA of the added mass owns one frequency and
-// IRF_CH pairs and its threads take the times in turn, so every cos/sin is
-// evaluated once per pair chunk. A serial sum over 1,000 times by one thread per
+// IRF_CH pairs and its threads take the times in turn: per pair chunk a cosine is
+// evaluated once and the sine of an inner time twice (as either end of a trapezium).
+// A serial sum over 1,000 times by one thread per
 // frequency was 1,580 us at 40 frequencies x 36 pairs (one CTA per chunk, each
 // step behind the last one's latency): now 17 us,
 // and K 66 to 24 us with 4 pairs a chunk instead of 16 (1,000 times).
