@@ -865,7 +865,8 @@ void solve_frequencies_impl(nemoh_ctx* c, int nomega, const double* omegas, int 
 // device bytes of the operand images of one item's FP64 updates, in a ragged batch
 // whose largest order is nmax
 size_t item_image_bytes(const nemoh_ctx* c, const BodyState& b, int nmax) {
-  return c->mode == NEMOH_B200_FP64 && nmax > LU_OUTER ? (b.nsymy + 1) * oz_bytes_per_system(nmax) : 0;
+  const bool tensor = c->mode == NEMOH_B200_FP64 && tc_enabled() && nmax > LU_OUTER;
+  return tensor ? (b.nsymy + 1) * oz_bytes_per_system(nmax) : 0;
 }
 
 // device bytes one item adds to a ragged batch whose largest order is nmax
