@@ -81,6 +81,10 @@ constexpr int OZ_EMIN = -250;
 // of 588 (0.8 M) 0.79 / 0.86, 2 of 894 (1.2 M) 1.00 / 1.04, 20 of 420 (1.7 M) 0.69 /
 // 0.66, 4 of 894 (2.3 M) 1.25 / 1.16, 2 of 1,430 (3.4 M) 2.09 / 1.86, 20 of 588
 // (4.2 M) 1.19 / 1.00, 1 of 2,380 (5.1 M) 4.05 / 3.21, 20 of 2,380 (101 M) 37.0 / 16.8.
+// Ragged: 1 of 1,400 with 19 of 200 (1.7 M after the first panel) 1.77 / 1.75, 2 of 1,100
+// with 20 of 200 (2.0 M) 1.50 / 1.46, 1 of 1,800 with 20 of 200 (2.9 M) 2.62 / 2.37, 3 of 1,000
+// with 6 of 500 (3.1 M) 1.49 / 1.36, 1 of 3,000 with 40 of 200 (8.5 M) 6.54 / 4.76, 4 of 2,600 with 8
+// of 1,200 and 12 of 400 (35 M) 13.6 / 7.6.
 constexpr double OZ_MIN_ENTRIES = 1.5e6;
 // Tiles of a full update (summed likewise) from which panel pairs are merged (four
 // per SM): the merged form reads and writes the trailing block once per pair, the
