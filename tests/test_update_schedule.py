@@ -37,7 +37,7 @@ def schedule():
 def _run(loads, plans, pick):
     fills, frees, content = [0] * SLOTS, [0] * SLOTS, [None] * SLOTS
     waits, held, at = [[0] * SLOTS, [0] * SLOTS], [set(), set()], [0, 0]
-    begun, full, drained = [0] * 4, [0] * 4, [0] * 4
+    begun, full, drained, summed = [0] * 4, [0] * 4, [0] * 4, [0] * 4
     made, loaded, pair = {}, 0, 0
 
     def load():
@@ -58,7 +58,8 @@ def _run(loads, plans, pick):
         accs = (2 * (pair % 2), 2 * (pair % 2) + 1)   # (0, 1), (2, 3), (0, 1), (2, 3) of a tile
         if any(full[a] == drained[a] for a in accs):
             return False
-        for a in accs:
+        for a in accs:   # a diagonal d has d + 1 products per chunk
+            assert summed[a] == 2 * (a + 1 if pair % 4 > 1 else 8 - a)
             drained[a] += 1
         pair += 1
         return True
@@ -72,6 +73,7 @@ def _run(loads, plans, pick):
         if first and drained[acc] < begun[acc] or any(fills[q] == waits[w][q] for q in slots):
             return False
         begun[acc] += first
+        summed[acc] = 1 if first else summed[acc] + 1
         for q in slots:
             waits[w][q] += 1
             assert waits[w][q] == fills[q] and q not in held[w]
